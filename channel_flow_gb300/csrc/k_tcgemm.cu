@@ -93,18 +93,23 @@ void fx_digits_host(double x, int e, double* dg, int np) {
 //   warp 0    producer: per K chunk of an item waits for a free stage, then
 //             moves the chunk's plane images with cp.async.bulk (completion
 //             counted in bytes on the stage's "full" barrier);
-//   warps 1-2 MMA issuers (4 planes: levels {0, 3} and {1, 2}, 5 of the 10
-//             products each; 3 planes: levels {0, 1} and {2}, 3 of the 6):
-//             wait for a free accumulator set (two sets of NP 64-column level
-//             accumulators, so one item's epilogue
-//             overlaps the next item's MMAs), per chunk wait for "full", issue
-//             their level MMAs per K16 slice (descriptors formed once per chunk,
-//             advanced by a constant per slice) and commit to the stage's
-//             "empty" barrier; after the last chunk they commit to "tfull";
-//   warps 3-10 epilogue: wait for "tfull", read the levels back with
+//   warp 1    MMA issuer (4 planes: 10 products per K16 slice, 3 planes: 6):
+//             waits for a free accumulator set (two sets of NP 64-column level
+//             accumulators, so one item's epilogue overlaps the next item's
+//             MMAs), per chunk waits for "full", issues the level MMAs of its
+//             K16 slices and commits to the stage's "empty" barrier; after the
+//             last chunk it commits to "tfull";
+//   warps 2-9 epilogue: wait for "tfull", read the levels back with
 //             tcgen05.ld (warp w reads TMEM lanes 32 (w % 4) .., columns
-//             32 ((w - 3) / 4) ..), release the set on "tempty" and form the
-//             outputs from the exact 64-bit level sum.
+//             32 ((w - 2) / 4) ..), release the set on "tempty" and form the
+//             outputs from the exact level sums.
+// What bounds it: a 128 x 64 x 16 MMA with both operands in shared memory
+// takes 48 clocks (measured: 32 + N / 4, the operand reads at 128 bytes per
+// clock; 32 of tensor work).  Issued warp-uniformly by one elected lane, with
+// the epilogue's stores in whole sectors, Z1 takes 56 us at 128 x 129 x 128
+// and 1.25 ms at 384 x 193 x 384 (90 us and 1.70 ms with two single-thread
+// issuers and one output row per epilogue thread), Z2 46 us and 0.63 ms (57
+// and 0.85), GL 31 us and 0.35 ms (39 and 0.50).
 // Every wait is bounded (1 s of wall time); a role that times out records
 // the failure, the others see it and stop, the producer waits for its copies
 // in flight and the MMA issuer drains its outstanding MMAs (both bounded)
@@ -113,9 +118,8 @@ void fx_digits_host(double x, int e, double* dg, int np) {
 // instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128, N = 64
 constexpr uint32_t IDESC_FX = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr int WS_STAGES = 4;
-constexpr int WS_MMA_WARPS = 2;  // issuers on disjoint level accumulators
 constexpr int WS_EPI_WARPS = 8;
-constexpr int WS_EPI0 = 1 + WS_MMA_WARPS;  // first epilogue warp
+constexpr int WS_EPI0 = 2;  // first epilogue warp (0: producer, 1: MMA issuer)
 constexpr int WS_THREADS = 32 * (WS_EPI0 + WS_EPI_WARPS);
 constexpr uint32_t WS_A_PLANE = 128u * TC_KC * 2u;
 constexpr uint32_t WS_B_PLANE = (uint32_t)FX_NT * TC_KC * 2u;
@@ -184,10 +188,23 @@ __device__ __forceinline__ double fx_out<double, 3>(const uint32_t* acc, int n) 
   return bits::scaled_i64(fx_level_sum<3>(acc), n);
 }
 
+// two adjacent outputs, stored together
+template <typename T>
+struct __align__(2 * sizeof(T)) Pair {
+  T a, b;
+};
+
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
+}
+
+// 1 in one lane of a converged warp, 0 in the others
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p;
 }
 
 __device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
@@ -208,10 +225,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
                                                               size_t ldc, int nfields, int* status,
                                                               long wait_ns, int skip_first) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t full[WS_STAGES], empty[WS_STAGES], tfull[2], tempty[2], drain[WS_MMA_WARPS], abar;
+  __shared__ __align__(8) uint64_t full[WS_STAGES], empty[WS_STAGES], tfull[2], tempty[2], drain, abar;
   __shared__ uint32_t tmem_base;
   __shared__ int s_fail;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   constexpr uint32_t SET_COLS = (uint32_t)FX_NT * NP;  // one accumulator set: NP levels
   const bool resident = ws_resident(plan);
   const int mt = (int)(blockIdx.x % plan.mtiles);
@@ -224,14 +241,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
     s_fail = 0;
     for (int i = 0; i < WS_STAGES; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[i])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&empty[i])), "r"(WS_MMA_WARPS));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&empty[i])));
     }
     for (int i = 0; i < 2; ++i) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&tfull[i])), "r"(WS_MMA_WARPS));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&tfull[i])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&tempty[i])), "r"(32 * WS_EPI_WARPS));
     }
-    for (int i = 0; i < WS_MMA_WARPS; ++i)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&drain[i])));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&drain)));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&abar)));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
@@ -243,7 +259,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
   volatile int* fail = &s_fail;
   const uint8_t* atile = aimg + (size_t)mt * plan.a_tile_bytes;
   if (warp == 0) {
@@ -287,86 +303,95 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
       if (resident && !mbar_wait(smem_u32(&abar), 0, wait_ns)) *fail = 7;
     }
   } else if (warp < WS_EPI0) {
-    // ---------------- MMA issuers ----------------
-    // the two issuers own disjoint level accumulators (see the selection
-    // below), with equal numbers of products per K16 slice
-    const int mw = warp - 1;
-    if (lane == 0) {
-      // K-adjacent core matrices: 16 (A, 128 rows) or 8 (B, 64 columns)
-      // groups of 8 rows x 16 bytes apart; adjacent 8-row groups 128 B apart.
-      // One K16 slice advances the start address by 2 core matrices: 256 / 128
-      // in the descriptor's 16-byte units.
-      const uint32_t lbo_a = 16u * 128u, lbo_b = 8u * 128u, sbo = 128u;
-      bool ok = !resident || mbar_wait(smem_u32(&abar), 0, wait_ns);
-      if (!ok) *fail = 3;
-      uint32_t g = 0, tc = 0;
-      for (long j = j0; ok && j < njobs && !*fail; j += jstep, ++tc) {
-        const uint32_t b = tc & 1u, tph = (tc >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&tempty[b]), tph ^ 1u, wait_ns)) {
-          *fail = 2;
+    // ---------------- MMA issuer ----------------
+    // The whole warp walks the loop and one elected lane issues, with every
+    // descriptor of a chunk a constant offset from two base values: in a
+    // branch of one thread each MMA took its operands through per-thread
+    // registers, and issuing, not the tensor pipe, set the MMA rate.
+    // K-adjacent core matrices: 16 (A, 128 rows) or 8 (B, 64 columns)
+    // groups of 8 rows x 16 bytes apart; adjacent 8-row groups 128 B apart.
+    // One K16 slice advances the start address by 2 core matrices: 256 / 128
+    // in the descriptor's 16-byte units.
+    const uint32_t lbo_a = 16u * 128u, lbo_b = 8u * 128u, sbo = 128u;
+    const uint32_t lead = elect_one();
+    bool ok = !resident || __all_sync(0xffffffffu, mbar_wait(smem_u32(&abar), 0, wait_ns));
+    if (!ok && lead) *fail = 3;
+    uint32_t g = 0, tc = 0;
+    for (long j = j0; ok && j < njobs; j += jstep, ++tc) {
+      if (__shfl_sync(0xffffffffu, *fail, 0)) break;
+      const uint32_t b = tc & 1u, tph = (tc >> 1) & 1u;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&tempty[b]), tph ^ 1u, wait_ns))) {
+        if (lead) *fail = 2;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t tacc = tmem + b * SET_COLS;
+      for (int ch = 0; ch < plan.nchunks; ++ch, ++g) {
+        const uint32_t s = g % WS_STAGES, ph = (g / WS_STAGES) & 1u;
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&full[s]), ph, wait_ns))) {
+          ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t tacc = tmem + b * SET_COLS;
-        for (int ch = 0; ch < plan.nchunks; ++ch, ++g) {
-          const uint32_t s = g % WS_STAGES, ph = (g / WS_STAGES) & 1u;
-          if (!mbar_wait(smem_u32(&full[s]), ph, wait_ns)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const int kc = plan.kc[ch];
-          const uint8_t* st = ring + (size_t)s * stage_bytes;
-          const uint8_t* sA = resident ? sAres + plan.a_chunk_off[ch] : st;
-          const uint32_t aplane = resident ? 128u * kc * 2u : WS_A_PLANE;
-          const uint8_t* sB = resident ? st : st + NP * WS_A_PLANE;
-          uint64_t da[NP], db[NP];
+        const int kc = plan.kc[ch];
+        const uint8_t* st = ring + (size_t)s * stage_bytes;
+        const uint8_t* sA = resident ? sAres + plan.a_chunk_off[ch] : st;
+        const uint32_t aplane = (resident ? 128u * kc * 2u : WS_A_PLANE) >> 4;
+        const uint8_t* sB = resident ? st : st + NP * WS_A_PLANE;
+        const uint64_t da = sdesc(smem_u32(sA), lbo_a, sbo), db = sdesc(smem_u32(sB), lbo_b, sbo);
+        if (lead) {
+          // products d_i e_(L-i) in rounds over i, so that consecutive MMAs
+          // accumulate into different levels (no read-after-write on one
+          // accumulator between neighbours); each level's first MMA (i = 0)
+          // comes in round 0
+          auto slice = [&](uint32_t k16, uint32_t first) {
 #pragma unroll
-          for (int pl = 0; pl < NP; ++pl) {
-            da[pl] = sdesc(smem_u32(sA + pl * aplane), lbo_a, sbo);
-            db[pl] = sdesc(smem_u32(sB + pl * WS_B_PLANE), lbo_b, sbo);
-          }
-          for (int k16 = 0; k16 < kc / 16; ++k16) {
-            const bool first = (ch == 0 && k16 == 0);
-            // products d_i e_(L-i) in rounds over i, so that consecutive MMAs
-            // accumulate into different levels (no read-after-write on one
-            // accumulator between neighbours); each level's first MMA (i = 0)
-            // comes in round 0
+            for (uint32_t i = 0; i < NP; ++i) {
 #pragma unroll
-            for (int i = 0; i < NP; ++i) {
-#pragma unroll
-              for (int L = i; L < NP; ++L) {
-                // issuer 0: levels {0, 3} (4 planes) or {0, 1} (3 planes)
-                if ((NP == 4 ? (L == 0 || L == 3) : L < 2) != (mw == 0)) continue;
-                const uint32_t accum = (first && i == 0) ? 0u : 1u;
+              for (uint32_t L = i; L < NP; ++L) {
+                const uint32_t accum = (i == 0 && first) ? 0u : 1u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tacc + (uint32_t)(L * FX_NT)),
-                    "l"(da[i] + (uint64_t)(k16 * 256)), "l"(db[L - i] + (uint64_t)(k16 * 128)), "r"(IDESC_FX),
-                    "r"(accum));
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tacc + L * FX_NT),
+                    "l"(da + (uint64_t)(i * aplane + k16 * 256)),
+                    "l"(db + (uint64_t)((L - i) * (WS_B_PLANE >> 4) + k16 * 128)), "r"(IDESC_FX), "r"(accum));
               }
             }
-          }
+          };
+          slice(0, ch == 0);
+          if (kc == TC_KC) slice(1, 0);
           mma_commit(smem_u32(&empty[s]));  // the stage is free once these MMAs have read it
         }
-        if (!ok) {
-          *fail = 3;
-          break;
-        }
-        mma_commit(smem_u32(&tfull[b]));
+        __syncwarp();
       }
-      // every MMA this thread issued has completed once "drain" arrives
-      mma_commit(smem_u32(&drain[mw]));
-      if (!mbar_wait(smem_u32(&drain[mw]), 0, wait_ns)) *fail = 4;
+      if (!ok) {
+        if (lead) *fail = 3;
+        break;
+      }
+      if (lead) mma_commit(smem_u32(&tfull[b]));
+      __syncwarp();
     }
+    // every MMA this warp issued has completed once "drain" arrives
+    if (lead) mma_commit(smem_u32(&drain));
+    __syncwarp();
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&drain), 0, wait_ns)) && lead) *fail = 4;
   } else {
     // ---------------- epilogue ----------------
-    const int q = warp & 3;                     // the TMEM lane quarter this warp may access
+    const int q = warp & 3;                         // the TMEM lane quarter this warp may access
     const int cbase = 32 * ((warp - WS_EPI0) / 4);  // its 32 of the 64 columns
-    const int row = q * 32 + lane;
-    const int m = mt * 128 + row;
-    const bool mrow = m < plan.mvalid;
-    const int fm = mrow ? aexp[m] : 0;
+    // A level is read in the 16x256b shape (two halves of 16 rows): a thread
+    // gets columns 2 (lane % 4), + 1 of every 8 in rows lane / 4 and + 8, so
+    // that the four lanes of a row store 32 (FP32) or 64 (FP64) consecutive
+    // bytes.  One row per thread (32x32b) made every 16-byte store of a warp
+    // touch 32 separate lines, and those stores, not the MMAs, set the time:
+    // about 140 clocks each.
+    const int rl = lane >> 2, cl = 2 * (lane & 3);
+    int fm[4];  // exponents of this thread's rows 8 i + rl of the quarter
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = mt * 128 + q * 32 + 8 * i + rl;
+      fm[i] = m < plan.mvalid ? aexp[m] : 0;
+    }
     uint32_t tc = 0;
     for (long j = j0; j < njobs; j += jstep, ++tc) {
       // decisions stay warp-uniform: tcgen05.ld needs the whole warp
@@ -382,15 +407,18 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
       OutT* out = outs.p[f];
+      // pairs of columns leave as one store when every pair is aligned
+      const bool paired = ((ldc | (size_t)plan.ncols) & 1u) == 0 &&
+                          (reinterpret_cast<uintptr_t>(out) & (2 * sizeof(OutT) - 1)) == 0;
 #pragma unroll
-      for (int g2 = 0; g2 < 2; ++g2) {
-        const int c0 = cbase + 16 * g2;
+      for (int hf = 0; hf < 2; ++hf) {  // rows 16 hf .. 16 hf + 15 of the quarter
         uint32_t r[NP][16];
 #pragma unroll
         for (int L = 0; L < NP; ++L) {
-          const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + b * SET_COLS + (uint32_t)(L * FX_NT + c0);
+          const uint32_t taddr =
+              tmem + ((uint32_t)(q * 32 + 16 * hf) << 16) + b * SET_COLS + (uint32_t)(L * FX_NT + cbase);
           asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+              "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
               "[%16];"
               : "=r"(r[L][0]), "=r"(r[L][1]), "=r"(r[L][2]), "=r"(r[L][3]), "=r"(r[L][4]), "=r"(r[L][5]),
                 "=r"(r[L][6]), "=r"(r[L][7]), "=r"(r[L][8]), "=r"(r[L][9]), "=r"(r[L][10]), "=r"(r[L][11]),
@@ -398,35 +426,33 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
               : "r"(taddr));
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;");
-        if (g2 == 1) {  // this warp's part of the set is in registers: release it
+        if (hf == 1) {  // this warp's part of the set is in registers: release it
           asm volatile("tcgen05.fence::before_thread_sync;");
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[b])) : "memory");
         }
-        int ec[16];
 #pragma unroll
-        for (int qq = 0; qq < 16; ++qq) ec[qq] = __shfl_sync(0xffffffffu, ecl, 16 * g2 + qq);
-        if (mrow) {
-          const size_t col = (size_t)nt * FX_NT + c0;
-          OutT* dst = out + (size_t)m * ldc + col;
-          OutT v[16];
+        for (int g8 = 0; g8 < 4; ++g8) {  // 8 columns each
+          const int e0 = __shfl_sync(0xffffffffu, ecl, 8 * g8 + cl), e1 = __shfl_sync(0xffffffffu, ecl, 8 * g8 + cl + 1);
+          const size_t col = (size_t)nt * FX_NT + cbase + 8 * g8 + cl;
 #pragma unroll
-          for (int qq = 0; qq < 16; ++qq) {
-            uint32_t acc[NP];
+          for (int i = 0; i < 2; ++i) {  // rows rl and rl + 8 of the half
+            const int m = mt * 128 + q * 32 + 16 * hf + 8 * i + rl;
+            if (m >= plan.mvalid) continue;
+            OutT v[2];
 #pragma unroll
-            for (int L = 0; L < NP; ++L) acc[L] = r[L][qq];
-            v[qq] = fx_out<OutT, NP>(acc, fm + ec[qq] - fx_shift<NP>());
-          }
-          // a thread's 16 outputs are consecutive in its row: 16-byte stores
-          // when the group is whole and aligned, element stores otherwise
-          if (col + 16 <= (size_t)plan.ncols && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-            uint4* d4 = reinterpret_cast<uint4*>(dst);
-            const uint4* v4 = reinterpret_cast<const uint4*>(v);
+            for (int k = 0; k < 2; ++k) {
+              uint32_t acc[NP];
 #pragma unroll
-            for (int k = 0; k < (int)(16 * sizeof(OutT) / 16); ++k) d4[k] = v4[k];
-          } else {
-#pragma unroll
-            for (int qq = 0; qq < 16; ++qq)
-              if (col + qq < (size_t)plan.ncols) dst[qq] = v[qq];
+              for (int L = 0; L < NP; ++L) acc[L] = r[L][4 * g8 + 2 * i + k];
+              v[k] = fx_out<OutT, NP>(acc, fm[2 * hf + i] + (k ? e1 : e0) - fx_shift<NP>());
+            }
+            OutT* dst = out + (size_t)m * ldc + col;
+            if (paired) {
+              if (col < (size_t)plan.ncols) *reinterpret_cast<Pair<OutT>*>(dst) = Pair<OutT>{v[0], v[1]};
+            } else {
+              if (col < (size_t)plan.ncols) dst[0] = v[0];
+              if (col + 1 < (size_t)plan.ncols) dst[1] = v[1];
+            }
           }
         }
       }

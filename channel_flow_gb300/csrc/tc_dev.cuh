@@ -24,19 +24,24 @@ __device__ __forceinline__ uint64_t gtimer() {
   return t;
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t phase) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(phase)
+      : "memory");
+  return ok;
+}
+
 // wait for the phase with parity `phase` to complete, at most limit_ns of
 // wall time (false on timeout)
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, long limit_ns = WAIT_NS) {
+  if (mbar_try(bar, phase)) return true;
   const uint64_t t0 = gtimer();
   for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(phase)
-        : "memory");
-    if (ok) return true;
+    if (mbar_try(bar, phase)) return true;
     if ((long)(gtimer() - t0) > limit_ns) return false;
   }
 }
