@@ -67,12 +67,13 @@ int upload_stage_twiddles(Handle* h) {
   const bool f32 = mixed_front(h);
   struct Tab {
     void** dst;
+    unsigned short** place;  // FP32 lines only
     const FftPlan* p;
     bool f32;
-  } tabs[] = {{&h->stw_py, &h->py, f32},
-              {&h->stw_px, &h->px, f32},
-              {(void**)&h->stw_py64, &h->py64, false},
-              {(void**)&h->stw_px64, &h->px64, false}};
+  } tabs[] = {{&h->stw_py, &h->place_py, &h->py, f32},
+              {&h->stw_px, &h->place_px, &h->px, f32},
+              {(void**)&h->stw_py64, nullptr, &h->py64, false},
+              {(void**)&h->stw_px64, nullptr, &h->px64, false}};
   for (const Tab& t : tabs) {
     if (!f32 && (t.dst == (void**)&h->stw_py64 || t.dst == (void**)&h->stw_px64)) continue;  // FP64 handle: py, px
     const int L = t.p->L;
@@ -85,6 +86,12 @@ int upload_stage_twiddles(Handle* h) {
     else
       fft_stage_twiddles<double>(*t.p, tw, reinterpret_cast<cd*>(host.data()));
     if (!cuda_ok(h, cudaMemcpy(*t.dst, host.data(), host.size(), cudaMemcpyHostToDevice), "stage twiddles"))
+      return CHF_E_CUDA;
+    if (!t.f32) continue;
+    std::vector<unsigned short> place(2 * (size_t)L, 0);
+    fft_place_tables(*t.p, place.data(), place.data() + L);
+    if (!*t.place && !cuda_ok(h, cudaMalloc((void**)t.place, 2 * place.size()), "stage twiddles")) return CHF_E_NOMEM;
+    if (!cuda_ok(h, cudaMemcpy(*t.place, place.data(), 2 * place.size(), cudaMemcpyHostToDevice), "stage twiddles"))
       return CHF_E_CUDA;
   }
   return CHF_OK;
@@ -181,7 +188,7 @@ static void release(chf_handle* h) {
   for (auto& p : h->mean) cudaFree(p);
   void* ptrs[] = {h->iapha, h->ibeta, h->t0, h->t2, h->t4, h->k2vals, h->xinv, h->xmean,
                   h->group_start, h->group_modes, h->tw_py, h->tw_px, h->tw_z2, h->tw_zm,
-                  h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->incm, h->incx, h->incr_exp, h->inc_items, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->scratch, h->dev_status, h->az1, h->az2,
+                  h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->place_py, h->place_px, h->incm, h->incx, h->incr_exp, h->inc_items, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->scratch, h->dev_status, h->az1, h->az2,
                   h->agl, h->bimg, h->wz32, h->wy32, h->lc64, h->aexp1, h->aexp2, h->aexp3, h->bexp, h->z2_tail, h->gl_tail};
   for (void* p : ptrs) cudaFree(p);
   for (auto& p : h->pending) {

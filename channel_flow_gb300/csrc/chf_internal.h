@@ -176,6 +176,9 @@ struct Handle {
   // (upload_stage_twiddles)
   void *stw_py = nullptr, *stw_px = nullptr;
   cd *stw_py64 = nullptr, *stw_px64 = nullptr;
+  // index tables of the in-place stages of py and px (mixed front; k_xy.cu,
+  // fft_place_tables): per plan L entries rev, L entries place
+  unsigned short *place_py = nullptr, *place_px = nullptr;
   cd *tw_py = nullptr, *tw_px = nullptr, *tw_z2 = nullptr, *tw_zm = nullptr;
   cf *twf_py = nullptr, *twf_px = nullptr;
 
@@ -323,6 +326,11 @@ int upload_stage_twiddles(Handle* h);
 bool xy_register_path(const Dims& d);
 int launch_yinv_fields(Handle* h, cf* wz, cf* wy, const cf* tw_py, int f0, int nf);
 int launch_xprod_yfwd(Handle* h, cf* wz, cf* wy, const cf* tw_py, const cf* tw_px);
+// in-place x / y transforms of FP32 lines (k_xy.cu)
+bool xy_in_place(const Dims& d);
+int launch_y_in_place(Handle* h, cf* wz, cf* wy, const FftPlan& py, const cf* stab, const unsigned short* rev,
+                      bool inverse);
+int launch_x_in_place(Handle* h, cf* wy, const FftPlan& px, const cf* stab, const unsigned short* tab);
 int launch_solve_fp64(Handle* h);
 int launch_solve_mean(Handle* h, cudaStream_t st);  // the (0,0) mode alone, on st
 int launch_solve_mixed(Handle* h);  // k_solve_mixed.cu

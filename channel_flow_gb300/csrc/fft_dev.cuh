@@ -33,6 +33,12 @@ struct FftPlan {
   // for r = 1 .. R - 1, jm = 0 .. Ns - 1 (L - 1 entries in all), so that the
   // threads of a stage read consecutive entries
   int twoff[16];
+  // in-place stages (k_xy.cu): division by LO = L / (Ns R) of each stage, the
+  // offset of stage st's Ns entries in the table of output digits
+  // (fft_place_tables), and the shift of the row swizzle
+  unsigned int lo_m[16];
+  int lo_s[16], roff[16];
+  int swz;
 };
 
 // m, s of the division by d (d >= 1) used in FftPlan: l = ceil(log2 d),
@@ -54,6 +60,14 @@ inline void fft_plan_divisors(FftPlan& p) {
     p.twoff[st] = off;
     off += (p.R[st] - 1) * p.Ns[st];
   }
+  off = 0;
+  for (int st = 0; st < p.nst; ++st) {
+    fft_divisor((unsigned int)(p.L / (p.Ns[st] * p.R[st])), &p.lo_m[st], &p.lo_s[st]);
+    p.roff[st] = off;
+    off += p.Ns[st];
+  }
+  const int last = p.nst > 0 ? p.R[p.nst - 1] : 1;
+  p.swz = last == 16 ? 4 : last == 8 ? 3 : last == 4 ? 2 : last == 2 ? 1 : 30;
 }
 
 __device__ __forceinline__ int fft_div(int n, unsigned int m, int s) {
@@ -380,6 +394,31 @@ inline void fft_stage_twiddles(const FftPlan& p, const V& tw, cplx<T>* out) {
         const auto& w = tw[(size_t)r * jm * step];
         out[p.twoff[st] + (r - 1) * Ns + jm] = cplx<T>{(T)w.re, (T)w.im};
       }
+  }
+}
+
+// Host side: the index tables of plan p for in-place stages.  A line's place
+// is a mixed-radix number with one digit per stage, the first stage's digit on
+// top (stride L / R[0]); stage st transforms its own digit where it stands,
+// so after the last stage place sum r_i L / (R_0 .. R_i) holds output
+// r_0 + R_0 r_1 + R_0 R_1 r_2 + ...
+//   rev[roff[st] + hi]  that sum over the digits before st for the places
+//                       whose upper digits form hi: the stage's twiddle index
+//   place[k]            the place of output k
+inline void fft_place_tables(const FftPlan& p, unsigned short* rev, unsigned short* place) {
+  for (int st = 0; st < p.nst; ++st)
+    for (int hi = 0; hi < p.Ns[st]; ++hi) {
+      int h = hi, jm = 0;
+      for (int i = st - 1; i >= 0; --i) {  // the last of the digits is the lowest
+        jm += (h % p.R[i]) * p.Ns[i];
+        h /= p.R[i];
+      }
+      rev[p.roff[st] + hi] = (unsigned short)jm;
+    }
+  for (int k = 0; k < p.L; ++k) {
+    int at = 0;
+    for (int i = 0; i < p.nst; ++i) at += (k / p.Ns[i] % p.R[i]) * (p.L / (p.Ns[i] * p.R[i]));
+    place[k] = (unsigned short)at;
   }
 }
 

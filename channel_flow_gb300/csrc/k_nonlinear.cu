@@ -801,6 +801,28 @@ int launch_xy(Handle* h, cplx<T>* wz, cplx<T>* wy, const cplx<T>* tw_py, const c
           h->err = "x/y transforms: radix above 9 in an FP64 plan";
           return CHF_E_INVALID;
         }
+  auto run_x = [&](int xr) {
+    return xr == 8 ? run_xprod<T, 8>(h, wy, px, stw_px)
+         : xr == 4 ? run_xprod<T, 4>(h, wy, px, stw_px)
+         : xr == 2 ? run_xprod<T, 2>(h, wy, px, stw_px)
+                   : run_xprod<T, 1>(h, wy, px, stw_px);
+  };
+  if constexpr (sizeof(T) == 4) {
+    // FP32 lines without a launch shape set: in place (k_xy.cu; y 2.05 -> 0.76
+    // and 1.05 -> 0.41 ms, x 3.27 -> 2.26 ms at 384 x 193 x 384).  FP64 lines,
+    // bound by the FP64 pipe, gain nothing there (x 8% slower at 128^3), and
+    // longer lines do not fit.  With fewer than four groups of 8 rows per SM
+    // the x kernel is one latency-bound wave, in which the two-buffer one's
+    // shorter index arithmetic wins (32^3: 11.0 against 12.8 us; 64 x 65 x 64,
+    // five groups: 25.9 against 25.3).
+    if (!h->tune.kxb && !h->tune.xr && xy_in_place(d)) {
+      int rc = launch_y_in_place(h, wz, wy, py, stw_py, h->place_py, true);
+      if (rc != CHF_OK) return rc;
+      const int xr = (long)d.MP * d.PY < 32L * h->num_sms ? pick_xr<T>(d) : 0;
+      rc = xr ? run_x(xr) : launch_x_in_place(h, wy, px, stw_px, h->place_px);
+      return rc == CHF_OK ? launch_y_in_place(h, wz, wy, py, stw_py, h->place_py, false) : rc;
+    }
+  }
   const int kxb = own && h->tune.kxb ? h->tune.kxb : pick_kxb<T>(d);
   const int xr = own && h->tune.xr ? h->tune.xr : pick_xr<T>(d);
   if (!kxb || !xr) {
@@ -818,10 +840,7 @@ int launch_xy(Handle* h, cplx<T>* wz, cplx<T>* wy, const cplx<T>* tw_py, const c
     if (!cuda_ok(h, cudaGetLastError(), "k_yinv")) return CHF_E_CUDA;
   }
   {
-    int rc = xr == 8 ? run_xprod<T, 8>(h, wy, px, stw_px)
-           : xr == 4 ? run_xprod<T, 4>(h, wy, px, stw_px)
-           : xr == 2 ? run_xprod<T, 2>(h, wy, px, stw_px)
-                     : run_xprod<T, 1>(h, wy, px, stw_px);
+    const int rc = run_x(xr);
     if (rc != CHF_OK) return rc;
   }
   {
