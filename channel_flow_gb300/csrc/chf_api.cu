@@ -110,7 +110,7 @@ std::vector<cd> twiddles(int L) {
 const char* const kKernelNames[K_COUNT] = {
     "k_zc2v", "k_yinv", "k_xprod", "k_yfwd", "k_zcurl", "k_solve", "k_diag",
     "k_tc_split_z1", "k_tc_gemm_z1", "k_tc_split_z2", "k_tc_gemm_z2", "k_curl", "k_tc_gemm_gl",
-    "k_meanfix", "k_inc_solve", "k_inc_recover", "k_solve_mean"};
+    "k_meanfix", "k_inc_solve", "k_inc_recover", "k_solve_mean", "k_xinv", "k_lamb", "k_zfwd", "k_zgl"};
 
 static cudaEvent_t take_event(Handle* h) {
   if (!h->event_pool.empty()) {
@@ -188,7 +188,7 @@ static void release(chf_handle* h) {
   for (auto& p : h->mean) cudaFree(p);
   void* ptrs[] = {h->iapha, h->ibeta, h->t0, h->t2, h->t4, h->k2vals, h->xinv, h->xmean,
                   h->group_start, h->group_modes, h->tw_py, h->tw_px, h->tw_z2, h->tw_zm,
-                  h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->place_py, h->place_px, h->incm, h->incx, h->incr_exp, h->inc_items, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->scratch, h->dev_status, h->az1, h->az2,
+                  h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->place_py, h->place_px, h->incm, h->incx, h->incr_exp, h->inc_items, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->wp, h->tf_image, h->scratch, h->dev_status, h->az1, h->az2,
                   h->agl, h->bimg, h->wz32, h->wy32, h->lc64, h->aexp1, h->aexp2, h->aexp3, h->bexp, h->z2_tail, h->gl_tail};
   for (void* p : ptrs) cudaFree(p);
   for (auto& p : h->pending) {
@@ -340,8 +340,10 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
     const size_t wz_elems = (size_t)6 * d.MP * d.modes();
     const size_t wy_elems = (size_t)6 * d.MP * d.PY * d.KX;
     if (!cuda_ok(h, cudaMalloc((void**)&h->wz, sizeof(cd) * wz_elems), "work alloc") ||
-        !cuda_ok(h, cudaMalloc((void**)&h->wy, sizeof(cd) * wy_elems), "work alloc"))
+        !cuda_ok(h, cudaMalloc((void**)&h->wy, sizeof(cd) * wy_elems), "work alloc") ||
+        (tf_xy(d) && !cuda_ok(h, cudaMalloc((void**)&h->wp, sizeof(double) * tf_phys_elems(d)), "work alloc")))
       return fail(CHF_E_NOMEM);
+    if (const int rc = setup_tf(h); rc != CHF_OK) return fail(rc);
   }
   if (!cuda_ok(h, cudaMalloc((void**)&h->dev_status, sizeof(int)), "status alloc") ||
       !cuda_ok(h, cudaMemsetAsync(h->dev_status, 0, sizeof(int), h->stream), "status init"))
@@ -386,10 +388,12 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
     if (!cuda_ok(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate")) return fail(CHF_E_CUDA);
   for (cudaEvent_t& e : h->ev_field)
     if (!cuda_ok(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate")) return fail(CHF_E_CUDA);
-  // FP64: k_zc2v, k_yinv, k_xprod, k_yfwd, k_zcurl, k_solve; mixed front:
+  // FP64: k_zc2v, k_yinv, k_xprod, k_yfwd, k_zcurl, k_solve (as digit
+  // products: x in three kernels, and k_zcurl as k_tf, k_curl64, k_tf and
+  // k_meanfix); mixed front:
   // two splits, three GEMMs, k_yinv_w, k_xprod_w, k_yfwd_w, k_curl,
   // k_meanfix; then k_solve, or k_inc_solve + k_inc_recover + the (0,0) mode
-  h->kernels_per_step = !mixed_front(h) ? 6 : increment_solve(h) ? 13 : 11;
+  h->kernels_per_step = !mixed_front(h) ? 6 + (tf_xy(d) ? 2 : 0) + (tf_z(d) ? 3 : 0) : increment_solve(h) ? 13 : 11;
   if (!cuda_ok(h, cudaStreamSynchronize(h->stream), "create sync")) return fail(CHF_E_CUDA);
   *out = h;
   return CHF_OK;

@@ -69,6 +69,17 @@ struct FxPlan {
   __host__ __device__ size_t bexp_stride() const { return (size_t)ntiles * FX_NT; }
 };
 
+// One dense transform of k_dft64.cu: line length L (the mirror's period), k
+// and n counts of its even (E) and odd (O) halves, their 16-wide k steps and
+// 8-wide output tiles, the matrix's power of two f, and its digit fragments.
+struct TfShape {
+  int L, k_e, k_o, n_e, n_o, ks_e, ks_o, tiles_e, tiles_o, f;
+};
+struct TfPlan {
+  TfShape s;
+  const void* mat;
+};
+
 template <typename T>
 struct Ptr8 {
   T* p[8];
@@ -185,6 +196,11 @@ struct Handle {
   // work buffers
   cd* wz = nullptr;   // 6 x [MP][KY][KX]  (values on the product grid)
   cd* wy = nullptr;   // 6 x [MP][PY][KX]  (after the spanwise transform)
+  double* wp = nullptr;  // 6 x [MP PY][PX] physical values (k_dft64.cu)
+  // FP64 transforms as digit products (k_dft64.cu): their plans, and the
+  // matrices' digit fragments followed by the tables they come from
+  TfPlan tf_z1{}, tf_gl{}, tf_z2{}, tf_yi{}, tf_yf{}, tf_xi{}, tf_xf{};
+  void* tf_image = nullptr;
   void* scratch = nullptr;  // reduction scratch (diagnostics)
   void* stats_buf = nullptr;  // chf_statistics: GL values of u, v, w + plane sums (first call)
   void* pres_buf = nullptr;   // chf_pressure: Lamb coefficients, right-hand sides, P (first call)
@@ -262,7 +278,7 @@ struct Handle {
 enum KernelId {
   K_ZC2V = 0, K_YINV, K_XPROD, K_YFWD, K_ZCURL, K_SOLVE, K_DIAG,
   K_SPLIT_Z1, K_GEMM_Z1, K_SPLIT_Z2, K_GEMM_Z2, K_CURL32, K_GEMM_GL, K_MEANFIX,
-  K_INC_SOLVE, K_INC_RECOVER, K_SOLVE_MEAN, K_COUNT
+  K_INC_SOLVE, K_INC_RECOVER, K_SOLVE_MEAN, K_XINV, K_LAMB64, K_ZFWD, K_GL64, K_COUNT
 };
 extern const char* const kKernelNames[K_COUNT];
 
@@ -326,6 +342,16 @@ int upload_stage_twiddles(Handle* h);
 bool xy_register_path(const Dims& d);
 int launch_yinv_fields(Handle* h, cf* wz, cf* wy, const cf* tw_py, int f0, int nf);
 int launch_xprod_yfwd(Handle* h, cf* wz, cf* wy, const cf* tw_py, const cf* tw_px);
+// FP64 transforms as exact digit products (k_dft64.cu)
+bool tf_z(const Dims& d);
+bool tf_xy(const Dims& d);
+size_t tf_phys_elems(const Dims& d);  // of wp
+int setup_tf(Handle* h);
+int launch_tf_c2v(Handle* h);
+int launch_tf_xy(Handle* h);
+int launch_tf_v2c(Handle* h, cd* const* hc);
+int launch_tf_curl(Handle* h);
+int launch_meanfix(Handle* h);  // k_mixed.cu
 // in-place x / y transforms of FP32 lines (k_xy.cu)
 bool xy_in_place(const Dims& d);
 int launch_y_in_place(Handle* h, cf* wz, cf* wy, const FftPlan& py, const cf* stab, const unsigned short* rev,

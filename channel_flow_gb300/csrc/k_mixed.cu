@@ -291,6 +291,16 @@ int setup_mixed(Handle* h) {
   return CHF_OK;
 }
 
+int launch_meanfix(Handle* h) {
+  const Dims& d = h->d;
+  cudaEvent_t ev;
+  prof_begin(h, K_MEANFIX, &ev);
+  k_meanfix<<<d.nch, 256, 0, h->stream>>>(h->f[F_U], h->f[F_W], h->mean[M_CL1N], h->mean[M_CL1NM1], h->mean[M_CL3N],
+                                          h->mean[M_CL3NM1], d.NZ, d.modes(), d.chm);
+  prof_end(h, K_MEANFIX, ev);
+  return cuda_ok(h, cudaGetLastError(), "k_meanfix") ? CHF_OK : CHF_E_CUDA;
+}
+
 int launch_nonlinear_mixed(Handle* h, const cudaEvent_t* field_ready) {
   const Dims& d = h->d;
   const long modes = d.modes(), cols = 2 * modes;
@@ -368,14 +378,7 @@ int launch_nonlinear_mixed(Handle* h, const cudaEvent_t* field_ready) {
   if ((rc = launch_tc_gemm_fx<double>(h, h->tgl, h->agl, h->aexp3, h->bimg, h->bexp, o2, 2, cols,
                                       K_GEMM_GL)) != CHF_OK)
     return rc;
-  {
-    cudaEvent_t ev;
-    prof_begin(h, K_MEANFIX, &ev);
-    k_meanfix<<<d.nch, 256, 0, h->stream>>>(h->f[F_U], h->f[F_W], h->mean[M_CL1N], h->mean[M_CL1NM1],
-                                            h->mean[M_CL3N], h->mean[M_CL3NM1], d.NZ, modes, d.chm);
-    prof_end(h, K_MEANFIX, ev);
-    if (!cuda_ok(h, cudaGetLastError(), "k_meanfix")) return CHF_E_CUDA;
-  }
+  if ((rc = launch_meanfix(h)) != CHF_OK) return rc;
   std::swap(h->f[F_U], h->f[F_RV]);
   std::swap(h->f[F_W], h->f[F_RG]);
   return CHF_OK;

@@ -860,20 +860,35 @@ int launch_xy(Handle* h, cplx<T>* wz, cplx<T>* wy, const cplx<T>* tw_py, const c
 template int launch_xy<double>(Handle*, cd*, cd*, const cd*, const cd*);
 template int launch_xy<float>(Handle*, cf*, cf*, const cf*, const cf*);
 
+// z inverse of the six fields (wz), then y, x, products and back (three
+// components in wz)
+static int launch_products_fp64(Handle* h) {
+  const Dims& d = h->d;
+  int rc;
+  if (tf_z(d)) {
+    rc = launch_tf_c2v(h);
+  } else {
+    const int zl = h->tune.zl_c2v ? h->tune.zl_c2v : pick_zl_c2v(d);
+    if (!zl) {
+      h->err = "z transforms: FFT length too large for the launch shapes";
+      return CHF_E_INVALID;
+    }
+    rc = zl == 8 ? run_zc2v<8>(h) : zl == 4 ? run_zc2v<4>(h) : run_zc2v<2>(h);
+  }
+  if (rc != CHF_OK) return rc;
+  return tf_xy(d) ? launch_tf_xy(h) : launch_xy<double>(h, h->wz, h->wy, h->tw_py, h->tw_px);
+}
+
 int launch_nonlinear_fp64(Handle* h) {
   const Dims& d = h->d;
-  // z inverse of the six fields u, v, w, ox, oy, oz
-  const int zl = h->tune.zl_c2v ? h->tune.zl_c2v : pick_zl_c2v(d);
   const int zc = h->tune.zl_curl ? h->tune.zl_curl : pick_zl_curl(d);
-  if (!zl || !zc) {
+  if (!tf_z(d) && !zc) {
     h->err = "z transforms: FFT length too large for the launch shapes";
     return CHF_E_INVALID;
   }
-  int rc = zl == 8 ? run_zc2v<8>(h) : zl == 4 ? run_zc2v<4>(h) : run_zc2v<2>(h);
+  int rc = launch_products_fp64(h);
   if (rc != CHF_OK) return rc;
-  rc = launch_xy<double>(h, h->wz, h->wy, h->tw_py, h->tw_px);
-  if (rc != CHF_OK) return rc;
-  rc = zc == 8 ? run_zcurl<8>(h) : zc == 4 ? run_zcurl<4>(h) : run_zcurl<2>(h);
+  rc = tf_z(d) ? launch_tf_curl(h) : zc == 8 ? run_zcurl<8>(h) : zc == 4 ? run_zcurl<4>(h) : run_zcurl<2>(h);
   if (rc != CHF_OK) return rc;
   std::swap(h->f[F_U], h->f[F_RV]);
   std::swap(h->f[F_W], h->f[F_RG]);
@@ -882,18 +897,16 @@ int launch_nonlinear_fp64(Handle* h) {
 
 // The Lamb vector of the current state (velocities and vorticities, as
 // after a solve) as Chebyshev coefficients hc = 3 x [NZ][modes], FP64; the
-// work buffers wz / wy must exist.  For the pressure (chf_pressure).
+// work buffers wz / wy (and wp) must exist.  For the pressure (chf_pressure).
 int launch_lamb_fp64(Handle* h, cd* hc) {
   const Dims& d = h->d;
-  const int zl = h->tune.zl_c2v ? h->tune.zl_c2v : pick_zl_c2v(d);
-  if (!zl) {
-    h->err = "z transforms: FFT length too large for the launch shapes";
-    return CHF_E_INVALID;
+  int rc = launch_products_fp64(h);
+  if (rc != CHF_OK) return rc;
+  if (tf_z(d)) {
+    cd* c[3] = {hc, hc + (size_t)d.NZ * d.modes(), hc + (size_t)2 * d.NZ * d.modes()};
+    return launch_tf_v2c(h, c);
   }
-  int rc = zl == 8 ? run_zc2v<8>(h) : zl == 4 ? run_zc2v<4>(h) : run_zc2v<2>(h);
-  if (rc != CHF_OK) return rc;
-  rc = launch_xy<double>(h, h->wz, h->wy, h->tw_py, h->tw_px);
-  if (rc != CHF_OK) return rc;
+  const int zl = h->tune.zl_c2v ? h->tune.zl_c2v : pick_zl_c2v(d);
   const size_t smem = zc2v_smem(d, zl);
   auto kern = zl == 8 ? k_zfwd<4, 8> : zl == 4 ? k_zfwd<4, 4> : k_zfwd<4, 2>;
   if (!set_smem(h, kern, smem)) return CHF_E_CUDA;
