@@ -188,7 +188,7 @@ static void release(chf_handle* h) {
   for (auto& p : h->mean) cudaFree(p);
   void* ptrs[] = {h->iapha, h->ibeta, h->t0, h->t2, h->t4, h->k2vals, h->xinv, h->xmean,
                   h->group_start, h->group_modes, h->tw_py, h->tw_px, h->tw_z2, h->tw_zm,
-                  h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->place_py, h->place_px, h->incm, h->incx, h->incr_exp, h->inc_items, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->wp, h->tf_image, h->scratch, h->dev_status, h->az1, h->az2,
+                  h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->place_py, h->place_px, h->incm, h->incx, h->incr_exp, h->inc_items, h->s64_mat, h->s64_exp, h->s64_ext, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->wp, h->tf_image, h->scratch, h->dev_status, h->az1, h->az2,
                   h->agl, h->bimg, h->wz32, h->wy32, h->lc64, h->aexp1, h->aexp2, h->aexp3, h->bexp, h->z2_tail, h->gl_tail};
   for (void* p : ptrs) cudaFree(p);
   for (auto& p : h->pending) {
@@ -372,15 +372,14 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
   if (upload_stage_twiddles(h) != CHF_OK) return fail(CHF_E_CUDA);
   int rc = setup_solver(h);
   if (rc != CHF_OK) return fail(rc);
-  if (mixed_front(h)) {
-    rc = setup_mixed(h);
-    if (rc == CHF_OK && increment_solve(h)) rc = setup_solver_mixed(h);
-    if (rc != CHF_OK) return fail(rc);
-    if (!cuda_ok(h, cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
-        !cuda_ok(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "cudaEventCreate") ||
-        !cuda_ok(h, cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming), "cudaEventCreate"))
-      return fail(CHF_E_CUDA);
-  }
+  if (mixed_front(h)) rc = setup_mixed(h);
+  if (rc == CHF_OK) rc = setup_inc_items(h);
+  if (rc == CHF_OK) rc = increment_solve(h) ? setup_solver_mixed(h) : setup_solve64(h);
+  if (rc != CHF_OK) return fail(rc);
+  if (!cuda_ok(h, cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
+      !cuda_ok(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "cudaEventCreate") ||
+      !cuda_ok(h, cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming), "cudaEventCreate"))
+    return fail(CHF_E_CUDA);
   if (!cuda_ok(h, cudaStreamCreateWithFlags(&h->copy_in, cudaStreamNonBlocking), "cudaStreamCreate") ||
       !cuda_ok(h, cudaStreamCreateWithFlags(&h->copy_out, cudaStreamNonBlocking), "cudaStreamCreate"))
     return fail(CHF_E_CUDA);
@@ -388,12 +387,13 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
     if (!cuda_ok(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate")) return fail(CHF_E_CUDA);
   for (cudaEvent_t& e : h->ev_field)
     if (!cuda_ok(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate")) return fail(CHF_E_CUDA);
-  // FP64: k_zc2v, k_yinv, k_xprod, k_yfwd, k_zcurl, k_solve (as digit
+  // FP64: k_zc2v, k_yinv, k_xprod, k_yfwd, k_zcurl (as digit
   // products: x in three kernels, and k_zcurl as k_tf, k_curl64, k_tf and
   // k_meanfix); mixed front:
   // two splits, three GEMMs, k_yinv_w, k_xprod_w, k_yfwd_w, k_curl,
-  // k_meanfix; then k_solve, or k_inc_solve + k_inc_recover + the (0,0) mode
-  h->kernels_per_step = !mixed_front(h) ? 6 + (tf_xy(d) ? 2 : 0) + (tf_z(d) ? 3 : 0) : increment_solve(h) ? 13 : 11;
+  // k_meanfix; then k_solve, or the modes' solve, k_inc_recover and the (0,0) mode
+  h->kernels_per_step = (mixed_front(h) ? 10 : 5 + (tf_xy(d) ? 2 : 0) + (tf_z(d) ? 3 : 0)) +
+                        (increment_solve(h) || solve64(h) ? 3 : 1);
   if (!cuda_ok(h, cudaStreamSynchronize(h->stream), "create sync")) return fail(CHF_E_CUDA);
   *out = h;
   return CHF_OK;

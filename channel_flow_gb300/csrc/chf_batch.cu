@@ -303,15 +303,15 @@ int build_stack(chf_batch* b, Stack& S) {
         return CHF_E_CUDA;
     }
     h->rec_df_rule = c0.rec_df_rule;  // the members' arithmetic
-    if (setup_inc_items(h) != CHF_OK) {
-      b->err = "class set-up: " + h->err;
-      return CHF_E_CUDA;
-    }
-    if (!ok(b, cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
-        !ok(b, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "cudaEventCreate") ||
-        !ok(b, cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming), "cudaEventCreate"))
-      return CHF_E_CUDA;
   }
+  if (setup_inc_items(h) != CHF_OK) {
+    b->err = "class set-up: " + h->err;
+    return CHF_E_CUDA;
+  }
+  if (!ok(b, cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
+      !ok(b, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "cudaEventCreate") ||
+      !ok(b, cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming), "cudaEventCreate"))
+    return CHF_E_CUDA;
   h->kernels_per_step = c0.kernels_per_step;
   h->uploaded = true;
   return ok(b, cudaDeviceSynchronize(), "class set-up") ? CHF_OK : CHF_E_CUDA;

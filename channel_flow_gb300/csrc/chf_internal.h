@@ -80,6 +80,17 @@ struct TfPlan {
   const void* mat;
 };
 
+// The four blocks (v even, v odd, omega even, omega odd) of k_solve64.cu as
+// 16 x 16 tiles: per parity the block size n, the rows and columns inside the
+// tiles, their tiles, and whether one last row and column stay outside; per
+// block its first strip of 16 rows, operator tile and staged operand tile.
+struct Sol64Shape {
+  int n[2], cols[2], tiles[2], ext[2];
+  int strip0[4], mat0[4], ext_off[4], staged[2][4];
+  int strips, staged_tiles, ext_stride;
+  size_t mat_stride;  // uint4 per k^2 group
+};
+
 template <typename T>
 struct Ptr8 {
   T* p[8];
@@ -158,6 +169,12 @@ struct Handle {
   // modes (n_inc_items[1] of them), then runs of at most 2 (n_inc_items[0])
   int2* inc_items = nullptr;
   int n_inc_items[2] = {0, 0};
+  // FP64 solve as digit products (k_solve64.cu), per k^2 group: digit tiles of
+  // M and A^-1, their rows' exponents, the rows and columns outside the tiles
+  Sol64Shape s64{};
+  uint4* s64_mat = nullptr;
+  short* s64_exp = nullptr;
+  double* s64_ext = nullptr;
   bool rec_df_rule = false;  // k_inc_recover's double-float form (setup_solver_mixed)
   double* xmean = nullptr;    // inverse of the (0,0) operator, NZ x NZ column-major
   int* group_start = nullptr; // nk2 + 1 (modes grouped by k^2)
@@ -234,7 +251,7 @@ struct Handle {
   // statistics
   int kernels_per_step = 0;
   cudaStream_t own_stream = nullptr;
-  // mixed path: the (0,0)-mode solve runs on a side stream beside the other
+  // the (0,0)-mode solve runs on a side stream beside the other
   // modes' solve (fork / join events on the handle's stream)
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -357,7 +374,11 @@ bool xy_in_place(const Dims& d);
 int launch_y_in_place(Handle* h, cf* wz, cf* wy, const FftPlan& py, const cf* stab, const unsigned short* rev,
                       bool inverse);
 int launch_x_in_place(Handle* h, cf* wy, const FftPlan& px, const cf* stab, const unsigned short* tab);
-int launch_solve_fp64(Handle* h);
+int launch_solve_fp64(Handle* h);  // k_solve.cu
+bool solve64(const Handle* h);     // k_solve64.cu
+int setup_solve64(Handle* h);
+int launch_solve64(Handle* h);
+int launch_recover(Handle* h, bool df);  // k_solve_mixed.cu: u, w, omega_x, omega_z from v, omega_y
 int launch_solve_mean(Handle* h, cudaStream_t st);  // the (0,0) mode alone, on st
 int launch_solve_mixed(Handle* h);  // k_solve_mixed.cu
 int launch_diagnostics(Handle* h, chf_diag* out);

@@ -43,14 +43,13 @@
 // forward 0.36 -> 0.25, z forward with curl and Gauss-Lobatto values 1.17 ->
 // 0.32; the errors against 64 bits of every array are equal or smaller (grids
 // of 4 to 192 points a side).
-#include <cuda_fp16.h>
-
 #include <algorithm>
 #include <climits>
 #include <cmath>
 #include <vector>
 
 #include "chf_internal.h"
+#include "digits64.cuh"
 
 namespace chf {
 
@@ -82,57 +81,15 @@ struct TfArgs {
   Dims d;
 };
 
-__device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// two digit bytes (as 128 + d) to FP16: 1024 + byte - 1152
-__device__ __forceinline__ uint32_t to_half2(uint32_t w, uint32_t sel) {
-  const uint32_t h = __byte_perm(w, 0x64646464u, sel);
-  const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&h), __half2half2(__ushort_as_half(0x6480)));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
-
-// x 2^(61 - e) rounded to an integer, |x| < 2^e, e = emax - 1022
-__device__ __forceinline__ long long fixed_of(uint32_t lo, uint32_t hi, int emax) {
-  const int ex = (int)((hi >> 20) & 0x7ffu);
-  if (ex == 0) return 0;  // zero (subnormals count as zero)
-  const int d = emax - ex;  // >= 0
-  if (d > 62) return 0;
-  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 8;
-  unsigned long long t = m >> d;
-  if (d > 0) t += (m >> (d - 1)) & 1ull;
-  return (int)hi < 0 ? -(long long)t : (long long)t;
-}
-
 // the digits of eight integers as FP16: word[p][j] holds digit p of x[2j], x[2j + 1]
 __device__ __forceinline__ void digit_halves(const long long* x, uint32_t (&word)[8][4]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const unsigned long long a = (unsigned long long)x[2 * j] + 0x8080808080808080ull;
-    const unsigned long long b = (unsigned long long)x[2 * j + 1] + 0x8080808080808080ull;
+    uint32_t w[8];
+    digit_pairs(x[2 * j], x[2 * j + 1], w);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {  // bytes 7..4, then 3..0
-      const uint32_t u = h ? (uint32_t)a : (uint32_t)(a >> 32), v = h ? (uint32_t)b : (uint32_t)(b >> 32);
-      const uint32_t top = __byte_perm(u, v, 0x7362), low = __byte_perm(u, v, 0x5140);  // bytes 2, 3 and 0, 1 of both
-      word[4 * h + 0][j] = to_half2(top, 0x4342);
-      word[4 * h + 1][j] = to_half2(top, 0x4140);
-      word[4 * h + 2][j] = to_half2(low, 0x4342);
-      word[4 * h + 3][j] = to_half2(low, 0x4140);
-    }
+    for (int p = 0; p < 8; ++p) word[p][j] = w[p];
   }
-}
-
-// hi 2^32 + lo += sum_p lev_p 256^(7-p), the eight level sums
-__device__ __forceinline__ void add_levels(const float (&lev)[8], long long& hi, long long& lo) {
-  int a[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) a[i] = __float2int_rn(lev[i]);
-  hi += (long long)(a[0] * 256 + a[1]) * 65536ll + (long long)(a[2] * 256 + a[3]);
-  lo += (long long)a[4] * 16777216ll + (long long)a[5] * 65536ll + ((long long)a[6] * 256ll + a[7]);
 }
 
 // t 2^n, the exponent added to the conversion's (n in the range where every
@@ -521,7 +478,6 @@ TfShape tf_shape(int L, int ke, int ko, int ne, int no) {
   return s;
 }
 
-constexpr size_t kMaxSmem = 227 * 1024;
 
 template <int MODE>
 int launch_tf(Handle* h, const TfPlan& p, const double* const* in, double* const* out, int nfields, long lines, int kid) {

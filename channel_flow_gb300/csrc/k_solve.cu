@@ -10,8 +10,7 @@
 // Design:
 //  * The operators depend on k^2 only (their alpha terms are switched off in
 //    the reference, tmpi = 0 at poiseuilleflow.f90:3363-3365, 3445), so one
-//    inverse is kept per distinct k^2 and modes are grouped by k^2: a CTA
-//    loads each inverse once for all modes that share it.
+//    inverse is kept per distinct k^2 and modes are grouped by k^2.
 //  * Collocation points z_p and z_{N-p} are mirror images and T_j, T_j'' and
 //    T_j'''' have parity (-1)^j there, so sums/differences of mirrored rows
 //    (and of the paired boundary rows) split each operator into an even-j and
@@ -157,8 +156,10 @@ __global__ void __launch_bounds__(INV_THREADS) k_invert(const double* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// Per-group solve: one CTA per distinct k^2 (plus one for the (0,0) mode),
-// modes of the group processed CH at a time.
+// Solve: one CTA per channel's (0,0) mode, then one per run of at most CH modes
+// of one k^2 group (setup_inc_items; the runs of a group share its inverse
+// through L2).  One CTA per group looping over its runs left small grids
+// waiting for the largest groups: 94 against 30 us at 32^3.
 // ---------------------------------------------------------------------------
 struct SolveArgs {
   cd *v, *oy, *u, *w, *ox, *oz;       // state (u, w hold the N^{n-1} histories on entry)
@@ -172,7 +173,7 @@ struct SolveArgs {
   FftPlan pz2;
   const cd* tw2;
   int nk2;
-  int g0;  // group of CTA 0 (nk2: the (0,0) mode alone)
+  const int2* items;  // {group, first mode index} of the CTAs after the (0,0) ones
   // constant flow rate: influence function phi of a unit mean pressure
   // gradient over one step, its bulk velocity, and the device word
   // flow = {target bulk velocity (0: off), last correction, bulk before, bulk after}
@@ -269,9 +270,10 @@ __global__ void __launch_bounds__(S_THREADS, 3) k_solve(const __grid_constant__ 
   }
   for (int j = threadIdx.x; j < NZ; j += blockDim.x) s.tj[j] = 2.0 * (double)j;
   __syncthreads();
-  const int g = blockIdx.x + a.g0;
-  const bool mean = (g >= a.nk2);
-  const int mch = mean ? g - a.nk2 : 0;      // the channel of a (0,0) group
+  const bool mean = (int)blockIdx.x < d.nch;
+  const int mch = mean ? (int)blockIdx.x : 0;  // the channel of a (0,0) mode
+  const int2 item = mean ? make_int2(a.nk2 + mch, 0) : a.items[(int)blockIdx.x - d.nch];
+  const int g = item.x;
   const long mean_mode = (long)mch * d.chm;  // its (0,0) mode
   const double dt = a.dt, re = a.group_re ? a.group_re[g] : a.re;
   double* const au0 = a.au0 + (size_t)mch * 2 * NZ;
@@ -284,10 +286,9 @@ __global__ void __launch_bounds__(S_THREADS, 3) k_solve(const __grid_constant__ 
   const double* X = a.xinv + (size_t)g * a.sl.stride;
   const SolveLayout& sl = a.sl;
   BlockOffsets bo = block_offsets(sl);
-  const int gs = mean ? 0 : a.group_start[g], ge = mean ? 2 : a.group_start[g + 1];
   const double c3 = 3.0 * dt / 2.0, c1 = dt / 2.0;
-  for (int base = gs; base < ge; base += CH) {
-    const int nm = min(CH, ge - base);
+  {
+    const int base = item.y, nm = mean ? CH : min(CH, a.group_start[g + 1] - base);
     // ---- A: load coefficients and explicit AB2 terms
     for (int t = tid; t < CH * NZ; t += blockDim.x) {
       int m = t / NZ, n = t % NZ;
@@ -479,8 +480,7 @@ __global__ void __launch_bounds__(S_THREADS, 3) k_solve(const __grid_constant__ 
         (m == 0 ? a.oz : a.ox)[(size_t)n * modes + mean_mode] =
             cd{sg * dslot(s, m, 0, NZ)[n], sg * dslot(s, m, 1, NZ)[n]};
       }
-      __syncthreads();
-      continue;
+      return;
     }
     for (int task = warp; task < nm * 2; task += S_WARPS) {  // Dv
       int m = task / 2, comp = task % 2;
@@ -526,7 +526,6 @@ __global__ void __launch_bounds__(S_THREADS, 3) k_solve(const __grid_constant__ 
       a.ox[idx] = cd{dwr + be * vv.im, dwi - be * vv.re};
       a.oz[idx] = cd{-dur - al * vv.im, -dui + al * vv.re};
     }
-    __syncthreads();
   }
 }
 
@@ -728,8 +727,8 @@ int setup_solver(Handle* h) {
   return CHF_OK;
 }
 
-// groups g0 .. nk2 (the last CTA is the (0,0) mode)
-static int launch_solve_from(Handle* h, int g0, cudaStream_t st) {
+// the (0,0) modes, and every other mode too unless mean_only
+static int launch_solve(Handle* h, bool mean_only, cudaStream_t st) {
   const Dims& d = h->d;
   SolveArgs a;
   a.v = h->f[F_V];
@@ -758,7 +757,7 @@ static int launch_solve_from(Handle* h, int g0, cudaStream_t st) {
   a.re = h->cfg.re;
   a.pz2 = h->pz2;
   a.tw2 = h->tw_z2;
-  a.g0 = g0;
+  a.items = h->inc_items + h->n_inc_items[1];
   a.phi = h->phi;
   a.ubphi = h->ubphi;
   a.flow = h->flow;
@@ -778,17 +777,34 @@ static int launch_solve_from(Handle* h, int g0, cudaStream_t st) {
                "k_solve smem"))
     return CHF_E_CUDA;
   cudaEvent_t ev;
-  prof_begin(h, g0 == 0 ? K_SOLVE : K_SOLVE_MEAN, &ev);
-  // groups g0 .. nk2 - 1 and the nch (0,0)-mode groups after them
-  kern<<<h->nk2 + h->d.nch - g0, S_THREADS, smem, st>>>(a);
-  prof_end(h, g0 == 0 ? K_SOLVE : K_SOLVE_MEAN, ev);
+  prof_begin(h, mean_only ? K_SOLVE_MEAN : K_SOLVE, &ev);
+  kern<<<d.nch + (mean_only ? 0 : h->n_inc_items[0]), S_THREADS, smem, st>>>(a);
+  prof_end(h, mean_only ? K_SOLVE_MEAN : K_SOLVE, ev);
   if (!cuda_ok(h, cudaGetLastError(), "k_solve")) return CHF_E_CUDA;
   return CHF_OK;
 }
 
-int launch_solve_fp64(Handle* h) { return launch_solve_from(h, 0, h->stream); }
+int launch_solve_mean(Handle* h, cudaStream_t st) { return launch_solve(h, true, st); }
 
-int launch_solve_mean(Handle* h, cudaStream_t st) { return launch_solve_from(h, h->nk2, st); }
+int launch_solve_fp64(Handle* h) {
+  if (!solve64(h)) return launch_solve(h, false, h->stream);
+  // the (0,0) mode touches only mode-0 entries and the mean arrays, which the
+  // kernels below neither write nor use: it runs beside them on the side
+  // stream (in order on the handle's stream while kernels are being timed)
+  cudaStream_t st = h->stream;
+  const bool fork = h->side_stream && !h->profiling;
+  int rc;
+  if (fork) {
+    if (!cuda_ok(h, cudaEventRecord(h->ev_fork, st), "solve fork") ||
+        !cuda_ok(h, cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0), "solve fork"))
+      return CHF_E_CUDA;
+    if ((rc = launch_solve_mean(h, h->side_stream)) != CHF_OK) return rc;
+    if (!cuda_ok(h, cudaEventRecord(h->ev_join, h->side_stream), "solve join")) return CHF_E_CUDA;
+  }
+  if ((rc = launch_solve64(h)) != CHF_OK || (rc = launch_recover(h, false)) != CHF_OK) return rc;
+  if (fork) return cuda_ok(h, cudaStreamWaitEvent(st, h->ev_join, 0), "solve join") ? CHF_OK : CHF_E_CUDA;
+  return launch_solve_mean(h, st);
+}
 
 int launch_diagnostics(Handle* h, chf_diag* out) {
   const Dims& d = h->d;

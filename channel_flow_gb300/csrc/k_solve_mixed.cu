@@ -748,10 +748,10 @@ int setup_solver_mixed(Handle* h) {
   if (!cuda_ok(h, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device), "SM count"))
     return CHF_E_CUDA;
   h->rec_df_rule = (4 * h->d.modes() + 31) / 32 >= 16L * nsm;
-  return setup_inc_items(h);
+  return CHF_OK;
 }
 
-// Work items of k_inc_solve, one CTA each: a k^2 group's modes in runs of at
+// Work items of k_inc_solve, k_solve and k_solve64, one CTA each: a k^2 group's modes in runs of at
 // most 4 (the first n_inc_items[1] entries) or 2 (the next n_inc_items[0]).
 // The runs of one group are adjacent in the list, so the CTAs that stream the
 // same operators run at the same time and share them through L2 instead of a
@@ -780,10 +780,20 @@ int setup_inc_items(Handle* h) {
   return CHF_OK;
 }
 
+int launch_recover(Handle* h, bool df) {
+  const long modes = h->d.modes();
+  auto kern = df ? k_inc_recover : k_inc_recover64;
+  cudaEvent_t ev;
+  prof_begin(h, K_INC_RECOVER, &ev);
+  kern<<<(unsigned)((4 * modes + RC_THREADS - 1) / RC_THREADS), RC_THREADS, 0, h->stream>>>(
+      h->f[F_V], h->f[F_OY], h->f[F_U], h->f[F_W], h->f[F_OX], h->f[F_OZ], h->iapha, h->ibeta, h->d);
+  prof_end(h, K_INC_RECOVER, ev);
+  return cuda_ok(h, cudaGetLastError(), "k_inc_recover") ? CHF_OK : CHF_E_CUDA;
+}
+
 int launch_solve_mixed(Handle* h) {
   const Dims& d = h->d;
   const int NZ = d.NZ;
-  const long modes = d.modes();
   const double dt = h->cfg.dt;
   cudaStream_t st = h->stream;
   cudaEvent_t ev;
@@ -829,16 +839,10 @@ int launch_solve_mixed(Handle* h) {
     prof_end(h, K_INC_SOLVE, ev);
     if (h->after_inc && !cuda_ok(h, cudaEventRecord(h->after_inc, st), "increment solve event")) return CHF_E_CUDA;
   }
-  {
-    // the double-float form where the grid gives it enough warps to hide its
-    // longer instruction stream, the FP64 form otherwise (fixed per grid)
-    const bool df = h->tune.rec_form >= 0 ? h->tune.rec_form == 1 : h->rec_df_rule;
-    auto kern = df ? k_inc_recover : k_inc_recover64;
-    prof_begin(h, K_INC_RECOVER, &ev);
-    kern<<<(unsigned)((4 * modes + RC_THREADS - 1) / RC_THREADS), RC_THREADS, 0, st>>>(
-        h->f[F_V], h->f[F_OY], h->f[F_U], h->f[F_W], h->f[F_OX], h->f[F_OZ], h->iapha, h->ibeta, d);
-    prof_end(h, K_INC_RECOVER, ev);
-  }
+  // the double-float form where the grid gives it enough warps to hide its
+  // longer instruction stream, the FP64 form otherwise (fixed per grid)
+  const int rc = launch_recover(h, h->tune.rec_form >= 0 ? h->tune.rec_form == 1 : h->rec_df_rule);
+  if (rc != CHF_OK) return rc;
   if (!cuda_ok(h, cudaGetLastError(), "mixed solve")) return CHF_E_CUDA;
   if (fork) return cuda_ok(h, cudaStreamWaitEvent(st, h->ev_join, 0), "solve join") ? CHF_OK : CHF_E_CUDA;
   // the (0,0) mode: the FP64 solve kernel, its last CTA only
