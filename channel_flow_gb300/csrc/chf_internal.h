@@ -87,7 +87,7 @@ struct TfPlan {
 struct Sol64Shape {
   int n[2], cols[2], tiles[2], ext[2];
   int strip0[4], mat0[4], ext_off[4], staged[2][4];
-  int strips, staged_tiles, ext_stride;
+  int strips, staged_tiles, ext_stride, pitch;
   size_t mat_stride;  // uint4 per k^2 group
 };
 

@@ -28,6 +28,17 @@
 // the increment to the coefficients.  Wall-normal sizes are mostly 2^a + 1, so
 // that the even blocks have 16 t + 1 rows: the last row and column stay out of
 // the tiles (a fifth of them at 129 points) and are plain FP64.
+//
+// What it measures, 128 x 129 x 128 (box 4 pi x 2 x 4/3 pi, 3077 runs): 331 us
+// (k_solve: 1314 with the recovery, which is 65 us here); DRAM 990 MB, 146 us
+// at 6763 GB/s.  No unit is full (matrix pipe 33%, FP64 28%, issue 37%):
+// 16 warps per SM wait on each other's latencies.  A strip's exponents, last
+// columns and coefficients come before its products or stay in shared memory
+// from the first part, because reading them after the products left three
+// DRAM latencies per strip in the open (405 us); three CTAs per SM spill
+// (474 us); operators brought to L2 during the first part change nothing
+// (332 us); with a one-tile read of the operators the time is 310 us, without
+// the products 288 us.
 #include <algorithm>
 
 #include "chf_internal.h"
@@ -40,6 +51,7 @@ namespace {
 constexpr int S64_MODES = 4;
 constexpr int S64_THREADS = 256;      // warps: 4 modes x 2 fields
 constexpr int S64_TILE = 520;         // words of a staged 16 x 8 tile: 8 planes x 32 lanes x 2, plus 8 to spread the banks
+constexpr int S64_NAN = 100000;
 constexpr int S64_BLOCK = 128;        // uint4 of a 16 x 16 operator tile: 4 per lane
 
 struct Sol64Args {
@@ -57,31 +69,46 @@ struct Sol64Args {
 };
 
 __device__ __forceinline__ int biased_exp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-__device__ __forceinline__ double power_of_two(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+// ta 2^a + tb 2^b: aligned and added as integers (|ta|, |tb| < 2^60), one
+// conversion, the exponent added to its bits
+__device__ __forceinline__ double increment(long long ta, int a, long long tb, int b) {
+  if (a >= S64_NAN / 2 || b >= S64_NAN / 2) return __longlong_as_double(0x7ff8000000000000ll);
+  const int m = max(a, b);
+  const long long t = (ta >> min(m - a, 63)) + (tb >> min(m - b, 63));
+  const double v = (double)t;
+  if (m < -960 || m > 900) return scalbn(v, m);
+  return t == 0 ? 0.0 : __hiloint2double(__double2hiint(v) + (m << 20), __double2loint(v));
+}
 
 template <int ITER>  // k pairs per lane: 32 ITER >= 8 tiles
 __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constant__ Sol64Args a) {
-  // staged digit tiles: [operand: coefficients, AB2 term][block][tile]
+  // staged digit tiles [operand: coefficients, AB2 term][block][tile], then
+  // the coefficients [block][mode][sh.pitch]
   extern __shared__ __align__(16) uint32_t dig[];
-  __shared__ double s_scale[2][4][S64_MODES];  // 2^(e - 66 + shift) of operand, block, mode
+  __shared__ int s_exp[2][4][S64_MODES];    // e - 66 + shift of operand, block, mode (S64_NAN: not finite)
   __shared__ int s_shift[2][4][S64_MODES];
   __shared__ double2 s_last[2][4][S64_MODES];  // the operand's value at the block's last column
+  __shared__ long s_mode[S64_MODES];
   const Sol64Shape& sh = a.s;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int2 it = a.items[blockIdx.x];
   const int grp = it.x, base = it.y, nm = min(S64_MODES, a.group_start[grp + 1] - base);
   const int N = a.N;
   const double* ext = a.ext + (size_t)grp * sh.ext_stride;
+  double2* s_c = reinterpret_cast<double2*>(dig + (size_t)sh.staged_tiles * S64_TILE);
+  const uint4* gmat = a.mat + (size_t)grp * sh.mat_stride;
   {
     // ---- the digits of one mode's field
     const int m = warp & 3, f = warp >> 2;
     const long mode = m < nm ? a.group_modes[base + m] : -1;
+    if (lane == 0 && f == 0) s_mode[m] = mode;
     const cd* C = (f == 0 ? a.v : a.oy) + (mode < 0 ? 0 : mode);
     const cd* H = (f == 0 ? a.rv : a.rg) + (mode < 0 ? 0 : mode);   // N^n
     const cd* Ho = (f == 0 ? a.u : a.w) + (mode < 0 ? 0 : mode);    // N^{n-1}
     const int wall = f == 0 ? 2 : 1;
     auto coef = [&](int j) { return mode >= 0 && j <= N ? C[(size_t)j * a.modes] : cd{0.0, 0.0}; };
-    auto term = [&](int p) {  // dt (3/2 N^n - 1/2 N^{n-1}) at point p
+    auto term = [&](int p) {  // half of dt (3/2 N^n - 1/2 N^{n-1}) at point p
       const cd h = H[(size_t)p * a.modes], o = Ho[(size_t)p * a.modes];
       return cd{a.c3 * h.re - a.c1 * o.re, a.c3 * h.im - a.c1 * o.im};
     };
@@ -89,8 +116,8 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
       e = o = cd{0.0, 0.0};
       if (mode < 0 || p < wall || p > N / 2) return;
       const cd x = term(p), y = term(N - p);
-      e = cd{0.5 * (x.re + y.re), 0.5 * (x.im + y.im)};
-      o = cd{0.5 * (x.re - y.re), 0.5 * (x.im - y.im)};
+      e = cd{x.re + y.re, x.im + y.im};
+      o = cd{x.re - y.re, x.im - y.im};
     };
     // x[set][i][comp of k, k + 1]: sets 0, 1 even / odd coefficients, 2, 3 even / odd term
     double x[4][ITER][4];
@@ -108,6 +135,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
           const bool in = k < sh.cols[t & 1];  // columns inside the tiles
           x[t][i][2 * h] = in ? y[t].re : 0.0;
           x[t][i][2 * h + 1] = in ? y[t].im : 0.0;
+          if (t < 2 && in) s_c[((2 * f + t) * S64_MODES + m) * sh.pitch + k] = make_double2(y[t].re, y[t].im);
         }
       }
 #pragma unroll
@@ -143,13 +171,13 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
         // |level sum| < 2^(66 + b) for sum |value| < 2^(e + b) (re and im together)
         const int b = max(0, 32 - __clz(sum) - 21);
         s_shift[op][blk][m] = 7 + b;
-        s_scale[op][blk][m] = e == 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(1.0, e - 1022 - 66 + 7 + b);
+        s_exp[op][blk][m] = e == 0x7ff ? S64_NAN : e - 1022 - 66 + 7 + b;
       }
     }
     // ---- the last row and column of a block of 16 t + 1
 #pragma unroll
     for (int par = 0; par < 2; ++par) {
-      if (!sh.ext[par]) continue;
+      if (!sh.ext[par] || mode < 0) continue;
       const int n = sh.n[par], blk = 2 * f + par, k = n - 1;
       const cd c = coef(2 * k + par);
       cd re, ro;
@@ -168,14 +196,14 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
           sr = fma(mm, x[par][i][2 * h], fma(xx, x[2 + par][i][2 * h], sr));
           si = fma(mm, x[par][i][2 * h + 1], fma(xx, x[2 + par][i][2 * h + 1], si));
         }
-      for (int o = 16; o > 0; o >>= 1) {
-        sr += __shfl_xor_sync(0xffffffffu, sr, o);
-        si += __shfl_xor_sync(0xffffffffu, si, o);
-      }
-      if (lane == 0 && mode >= 0) {
-        sr = fma(rowm[k], c.re, fma(rowx[k], r.re, sr));
-        si = fma(rowm[k], c.im, fma(rowx[k], r.im, si));
-        ((f == 0 ? a.v : a.oy) + mode)[(size_t)(2 * k + par) * a.modes] = cd{c.re + sr, c.im + si};
+      // the lower half-warp sums the real parts, the upper one the imaginary
+      const bool up = lane >= 16;
+      double sum = (up ? si : sr) + __shfl_xor_sync(0xffffffffu, up ? sr : si, 16);
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((lane & 15) == 0) {
+        const double cc = up ? c.im : c.re;
+        sum = fma(rowm[k], cc, fma(rowx[k], up ? r.im : r.re, sum));
+        reinterpret_cast<double*>((f == 0 ? a.v : a.oy) + mode + (size_t)(2 * k + par) * a.modes)[up] = cc + sum;
       }
       if (lane == 0) {
         s_last[0][blk][m] = make_double2(c.re, c.im);
@@ -186,18 +214,27 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
   __syncthreads();
   // ---- strips of 16 rows through M and X
   const int row = lane >> 2, q = lane & 3;  // the lane's rows row, row + 8 and its mode
-  const long mode = q < nm ? a.group_modes[base + q] : -1;
-  const uint4* gmat = a.mat + (size_t)grp * sh.mat_stride + lane;
-  const short* gexp = a.exps + (size_t)grp * sh.strips * 32;
+  const long mode = s_mode[q];
+  const short4* gexp = reinterpret_cast<const short4*>(a.exps) + (size_t)grp * sh.strips * 8 + row;
   for (int s = warp; s < sh.strips; s += S64_THREADS / 32) {
     int blk = 0;
     while (blk < 3 && s >= sh.strip0[blk + 1]) ++blk;
     const int i = s - sh.strip0[blk], par = blk & 1, T = sh.tiles[par], n = sh.n[par];
-    const uint4* mp = gmat + (size_t)(sh.mat0[blk] + 2 * T * i) * S64_BLOCK;
-    double dr[2] = {0.0, 0.0}, di[2] = {0.0, 0.0};  // increments of rows row, row + 8
+    const uint4* mp = gmat + lane + (size_t)(sh.mat0[blk] + 2 * T * i) * S64_BLOCK;
+    long long prod[2][4];  // M c and X r of (row, re), (row, im), (row + 8, re), (row + 8, im)
     uint4 w[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) w[c] = __ldg(mp + c * 32);
+    const short4 rexp = gexp[s * 8];  // of M and X in row, of M and X in row + 8
+    double colm[2] = {0.0, 0.0}, colx[2] = {0.0, 0.0};  // the last column of M and X
+    if (sh.ext[par]) {
+      const double* col = ext + sh.ext_off[blk] + 2 * n + 16 * i + row;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        colm[h] = col[8 * h];
+        colx[h] = col[n - 1 + 8 * h];
+      }
+    }
 #pragma unroll 1
     for (int op = 0; op < 2; ++op) {
       float acc[8][4];
@@ -226,16 +263,14 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
         }
       }
       const int sft = s_shift[op][blk][q];
-      const double scale = s_scale[op][blk][q];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const float lev[8] = {acc[0][c], acc[1][c], acc[2][c], acc[3][c], acc[4][c], acc[5][c], acc[6][c], acc[7][c]};
         long long hi = 0, lo = 0;
         add_levels(lev, hi, lo);
         const long long t = (hi << (32 - sft)) + ((lo + (1ll << (sft - 1))) >> sft);
-        const double z = (double)t * (scale * power_of_two(gexp[s * 32 + op * 16 + row + 8 * (c >> 1)]));
-        if (c & 1) di[c >> 1] += z;
-        else dr[c >> 1] += z;
+        if (op == 0) prod[0][c] = t;
+        else prod[1][c] = t;
       }
     }
     if (mode < 0) continue;
@@ -244,16 +279,16 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
     for (int h = 0; h < 2; ++h) {
       const int r = 16 * i + row + 8 * h;
       if (r >= sh.cols[par]) continue;  // tile rows past the block
+      const int em = s_exp[0][blk][q] + (h ? rexp.z : rexp.x), ex = s_exp[1][blk][q] + (h ? rexp.w : rexp.y);
+      double dr = increment(prod[0][2 * h], em, prod[1][2 * h], ex);
+      double di = increment(prod[0][2 * h + 1], em, prod[1][2 * h + 1], ex);
       if (sh.ext[par]) {
-        const double* colm = ext + sh.ext_off[blk] + 2 * n;
-        const double mm = colm[r], xx = colm[n - 1 + r];
         const double2 c = s_last[0][blk][q], t = s_last[1][blk][q];
-        dr[h] = fma(mm, c.x, fma(xx, t.x, dr[h]));
-        di[h] = fma(mm, c.y, fma(xx, t.y, di[h]));
+        dr = fma(colm[h], c.x, fma(colx[h], t.x, dr));
+        di = fma(colm[h], c.y, fma(colx[h], t.y, di));
       }
-      cd* o = dst + (size_t)(2 * r + par) * a.modes;
-      const cd c = *o;
-      *o = cd{c.re + dr[h], c.im + di[h]};
+      const double2 c = s_c[(blk * S64_MODES + q) * sh.pitch + r];
+      dst[(size_t)(2 * r + par) * a.modes] = cd{c.x + dr, c.y + di};
     }
   }
 }
@@ -337,7 +372,8 @@ __global__ void __launch_bounds__(256) k_digits_solve64(const double* __restrict
   __syncthreads();
   // a row's power of two; entries 2^-600 below are zero, rows of zeros take 0
   if (tid < 32)
-    exps[((size_t)g * sh.strips + s) * 32 + tid] = (short)(s_e[tid >> 4][tid & 15] ? s_e[tid >> 4][tid & 15] - 1022 : 0);
+    exps[(((size_t)g * sh.strips + s) * 8 + (tid & 7)) * 4 + 2 * ((tid >> 3) & 1) + (tid >> 4)] =
+        (short)(s_e[tid >> 4][tid & 15] ? s_e[tid >> 4][tid & 15] - 1022 : 0);
   uint4* out = mat + (size_t)g * sh.mat_stride + (size_t)(sh.mat0[blk] + 2 * T * i) * S64_BLOCK + lane;
   for (int t = warp; t < 2 * T; t += 8) {
     const int op = t / T, kt = t - op * T;
@@ -392,6 +428,8 @@ Sol64Shape solve64_shape(int N) {
     if (s.ext[par]) ext += 4 * s.n[par];
   }
   s.strips = strip;
+  // rows 1 and 2 apart and modes apart by 2 (mod 8) of the 16-byte banks
+  s.pitch = (s.n[0] + 5) / 8 * 8 + 2;
   s.staged_tiles = staged;
   s.mat_stride = (size_t)mat * S64_BLOCK;
   s.ext_stride = std::max(1, ext);
@@ -401,10 +439,10 @@ Sol64Shape solve64_shape(int N) {
 // CHF_FP64 takes this path where k_solve's CTAs (runs of 2 modes and the (0,0)
 // mode) would be more than one per SM: below that both are bound by latency,
 // and k_solve is one kernel instead of three and needs no further set-up.
-// Whole steps, this path against k_solve: 32 x 17 x 32 85 / 88 us, 32^3 118 /
-// 118 (216 / 241 with three such channels at a time), 64 x 65 x 64 462 / 544,
-// 128 x 129 x 128 3316 / 4117; with fewer CTAs than SMs 16 x 65 x 16 131 / 125,
-// 16 x 65 x 4 121 / 115, 24 x 21 x 12 78 / 80.
+// Whole steps, this path against k_solve, on the same transforms: 32 x 17 x 32
+// 85 / 88 us, 32^3 112 / 118 (216 / 241 with three such channels at a time),
+// 64 x 65 x 64 462 / 544, 128 x 129 x 128 2717 / 3600; with fewer CTAs than
+// SMs 16 x 65 x 16 131 / 125, 16 x 65 x 4 121 / 115, 24 x 21 x 12 78 / 80.
 // CHF_MIXED_F64SOLVE stays with k_solve: its FP32 front turns any change of
 // the state's last bit into another rounding of the next step.
 bool solve64(const Handle* h) {
@@ -456,9 +494,9 @@ int launch_solve64(Handle* h) {
   a.N = h->d.N;
   a.NZ = h->d.NZ;
   a.modes = h->d.modes();
-  a.c3 = 1.5 * h->cfg.dt;
-  a.c1 = 0.5 * h->cfg.dt;
-  const size_t smem = sizeof(uint32_t) * S64_TILE * (size_t)s.staged_tiles;
+  a.c3 = 0.75 * h->cfg.dt;
+  a.c1 = 0.25 * h->cfg.dt;
+  const size_t smem = sizeof(uint32_t) * S64_TILE * (size_t)s.staged_tiles + sizeof(double2) * 4 * S64_MODES * s.pitch;
   auto kern = std::max(s.tiles[0], s.tiles[1]) <= 4 ? k_solve64<1> : k_solve64<2>;
   if (!cuda_ok(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "k_solve64 smem"))
     return CHF_E_CUDA;
