@@ -125,10 +125,9 @@ struct Tuning {
   int xr = 0;       // (plane, y) rows per CTA of the shared-memory x transform
   int zl_c2v = 0;   // modes per CTA of the FP64 z transform to the product grid
   int zl_curl = 0;  // modes per CTA of the FP64 z transform + curl
-  int inc_mch = 4;  // modes per CTA (work item) of the increment solve (2 or 4)
+  int inc_mch = 0;  // modes per CTA (work item) of the increment solve (2 or 4; 0: inc_modes)
   int inc_cb = 4;   // matrix columns per load batch of the increment solve (2..4)
   int inc_rpt = 1;  // rows per thread of the increment solve (1 or 2; 2 with 2 or 3 columns)
-  int inc_wide = 1; // one row per thread: every block row in one pass (1) or loop (0)
   // arithmetic of k_inc_recover (not searched by the autotuner): -1 the
   // handle's rule, 0 FP64, 1 double-float (2^-44 relative)
   int rec_form = -1;
@@ -380,6 +379,7 @@ int setup_solve64(Handle* h);
 int launch_solve64(Handle* h);
 int launch_recover(Handle* h, bool df);  // k_solve_mixed.cu: u, w, omega_x, omega_z from v, omega_y
 int launch_solve_mean(Handle* h, cudaStream_t st);  // the (0,0) mode alone, on st
+int inc_modes(const Handle* h);  // modes per CTA of k_inc_solve
 int launch_solve_mixed(Handle* h);  // k_solve_mixed.cu
 int launch_diagnostics(Handle* h, chf_diag* out);
 

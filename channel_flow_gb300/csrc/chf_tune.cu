@@ -124,11 +124,11 @@ std::string describe(const Handle* h, double ms_rule, double ms_best) {
   char buf[512];
   std::snprintf(buf, sizeof buf,
                 "fft radices py %s px %s pz2 %s pzm %s; kxb %d xr %d zl_c2v %d zl_curl %d; "
-                "increment solve %d modes x %d columns x %d rows per thread%s, %s recovery; step %.4f ms "
+                "increment solve %d modes x %d columns x %d rows per thread, %s recovery; step %.4f ms "
                 "(rules %.4f ms)",
                 radix_string(h->py).c_str(), radix_string(h->px).c_str(), radix_string(h->pz2).c_str(),
                 radix_string(h->pzm).c_str(), h->tune.kxb, h->tune.xr, h->tune.zl_c2v, h->tune.zl_curl,
-                h->tune.inc_mch, h->tune.inc_cb, h->tune.inc_rpt, h->tune.inc_wide ? "" : " (288-thread blocks)",
+                inc_modes(h), h->tune.inc_cb, h->tune.inc_rpt,
                 (h->tune.rec_form >= 0 ? h->tune.rec_form == 1 : h->rec_df_rule) ? "double-float" : "FP64", ms_best,
                 ms_rule);
   return buf;
@@ -240,21 +240,16 @@ int chf_autotune(chf_handle* h, int reps) {
   try_knob([&](const FftPlan& p) { h->pz2 = p; }, with_current(h->pz2, plan_candidates(make_plan(2 * d.N))));
   if (increment_solve(h)) {
     struct IncMap {
-      int mch, cb, rpt, wide;
+      int mch, cb, rpt;
     };
-    std::vector<IncMap> maps{{h->tune.inc_mch, h->tune.inc_cb, h->tune.inc_rpt, h->tune.inc_wide}};
-    const SolveLayout& sl = h->sl;
-    const bool long_blocks = sl.ne_v + sl.no_v + sl.ne_w + sl.no_w > 288;  // the one-row block loops
-    for (int wide : {1, 0}) {
-      if (wide == 0 && !long_blocks) continue;
-      for (int mch : {4, 2})
-        for (int cb : {4, 3, 2}) maps.push_back({mch, cb, 1, wide});
-    }
+    std::vector<IncMap> maps{{h->tune.inc_mch, h->tune.inc_cb, h->tune.inc_rpt}};
     for (int mch : {4, 2})
-      for (int cb : {3, 2}) maps.push_back({mch, cb, 2, 1});
+      for (int cb : {4, 3, 2}) maps.push_back({mch, cb, 1});
+    for (int mch : {4, 2})
+      for (int cb : {3, 2}) maps.push_back({mch, cb, 2});
     try_knob(
         [&](const IncMap& m) {
-          h->tune.inc_mch = m.mch, h->tune.inc_cb = m.cb, h->tune.inc_rpt = m.rpt, h->tune.inc_wide = m.wide;
+          h->tune.inc_mch = m.mch, h->tune.inc_cb = m.cb, h->tune.inc_rpt = m.rpt;
         },
         maps);
   }
@@ -309,8 +304,7 @@ int chf_set_launch_shape(chf_handle* h, const char* name, int value) {
     if (value != 1 && value != 2) return bad("1 or 2 rows per thread");
     t.inc_rpt = value;
   } else if (n == "inc_wide") {
-    if (value != 0 && value != 1) return bad("0 or 1");
-    t.inc_wide = value;
+    if (value != 0 && value != 1) return bad("0 or 1");  // one pass holds every row: nothing to choose
   } else if (n == "recover_form") {
     if (value < -1 || value > 1) return bad("-1 (rule), 0 (FP64) or 1 (double-float)");
     t.rec_form = value;

@@ -18,8 +18,8 @@
 // M = A^-1 (B - A) = A^-1 B - I maps coefficients to coefficients and has no
 // such cancellation (its rows sum to within ~10x of the result; at 128^3
 // the largest row sum is ~150, the median ~2).  A step is then
-//   k_inc_solve    one CTA per run of at most 4 (or 2) modes of one k^2
-//                  group: delta = M c (compensated FP32 on (hi, lo) splits of
+//   k_inc_solve    one CTA per field and run of at most 4 (or 2) modes of one
+//                  k^2 group: delta = M c (compensated FP32 on (hi, lo) splits of
 //                  M and c, summed against a power-of-two offset) + A^-1 r
 //                  (FP32), x = c + delta in FP64
 //   k_inc_recover  u, w, omega_x, omega_z from v and omega_y (getvelocityandvorticity,
@@ -41,7 +41,6 @@ namespace chf {
 
 namespace {
 
-constexpr int MV_THREADS = 288;  // threads over the 2 NZ rows of one group's four blocks
 // modes per CTA (MCH), matrix columns per load batch (CB) and rows per thread
 // of k_inc_solve are template parameters: the defaults 4, 4 and 1, others
 // picked by the autotuner (chf_tune.cu)
@@ -128,10 +127,11 @@ __global__ void __launch_bounds__(128) k_incr_rowexp(const float2* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// k_inc_solve: one CTA per work item, up to MCH modes of one k^2 group (mean
-// excluded; setup_inc_items).  Per mode the CTA stages in shared memory
-//   * the coefficients c of v and omega_y as (hi, lo) floats, ordered as the
-//     four blocks' columns (v even j, v odd j, omega even j, omega odd j);
+// k_inc_solve: one CTA per work item (up to MCH modes of one k^2 group, mean
+// excluded; setup_inc_items) and field (v, omega_y).  Per mode the CTA stages
+// in shared memory
+//   * the field's coefficients c as (hi, lo) floats, ordered as the columns of
+//     its two blocks (even j, odd j);
 //   * the AB2 term r = dt (3/2 N^n - 1/2 N^{n-1}) at the Gauss-Lobatto
 //     points, folded (even rows 1/2 (r_p + r_{N-p}), odd rows
 //     1/2 (r_p - r_{N-p}), p = row) with the wall rows zero, as floats;
@@ -149,6 +149,19 @@ __global__ void __launch_bounds__(128) k_incr_rowexp(const float2* __restrict__ 
 // delta = (S - sigma) + C with S - sigma exact: M c to about
 // 2^-38 sum_c |M_rc| max|c| (sigma is at most 2^5 of that; the dropped
 // parts are 2^-43 of sigma), X r to FP32 rounding.
+//
+// The work splits by field because nothing of a CTA's staging (gathers of
+// 16 bytes a lane, bound by latency and by the L1's tags) overlaps its own
+// products: more and smaller CTAs per SM overlap each other's.  One CTA for
+// both fields / this kernel: 15.2 / 12.4 us at 32 x 33 x 32, 178 / 160 at
+// 160 x 97 x 120, 214 / 209 at 128 x 129 x 128, 3226 / 3089 at 384 x 193 x 384
+// (12.0 GB, 57% of 6763 GB/s).  Parts switched off there, of 3226: without the
+// staging 2505, without the products 879, every group reading the same 32
+// operators 3091, without the arithmetic 2881: no one resource is full, the
+// times add.  Not faster: the operators through a ring of bulk copies in
+// shared memory (3370 to 4490), brought to L2 ahead (3137 and, at 128 x 129 x
+// 128, 207 against 202 of the same shape), the gathers of all modes asked for
+// together (3385), warp reductions for the exponents (3129 against 3089).
 // ---------------------------------------------------------------------------
 struct __align__(16) CoefHL {
   float hr, hi, lr, li;  // high and low parts of the real and imaginary parts
@@ -173,33 +186,22 @@ __device__ __forceinline__ void sig_mac2(f32x2 mh, f32x2 ml, f32x2 ch, f32x2 cl,
 }
 
 // Rows of one pass of k_inc_solve for NM staged modes: each thread owns RPT
-// adjacent rows of one of the four blocks (v even, v odd, omega even,
-// omega odd), so that every staged coefficient and AB2 value read from
-// shared memory serves RPT rows.  The staged values of entry e of mode q sit
+// adjacent rows of one of the field's two blocks (even, odd), so that every
+// staged coefficient and AB2 value read from shared memory serves RPT rows.  The staged values of entry e of mode q sit
 // at e MS + q (MS = the kernel's modes per CTA), so one address per column
 // reaches every mode by constant offsets; the matrix columns are walked by
 // element offsets advanced per batch, and only the last batch checks the
 // column count.  The arithmetic of a row does not depend on RPT.
 template <int NM, int MS, int CB, int RPT>
-__device__ __forceinline__ void inc_rows(cd* __restrict__ v, cd* __restrict__ g, const float2* __restrict__ Mg,
-                                         const float* __restrict__ Xg, const SolveLayout& sl,
-                                         const BlockOffsets& bo, int NZ, long modes, const cd* Cd,
-                                         const CoefHL* Cs, const float2* Rs, const int* s_mode,
+__device__ __forceinline__ void inc_rows(cd* __restrict__ dst, const float2* __restrict__ Mg,
+                                         const float* __restrict__ Xg, int ne, int no, int odd, int NZ, long modes,
+                                         const cd* Cd, const CoefHL* Cs, const float2* Rs, const int* s_mode,
                                          const signed char* __restrict__ rexp, const int* s_cexp) {
-  const int nev = sl.ne_v, nov = sl.no_v, new_ = sl.ne_w, now_ = sl.no_w;
-  // slots (groups of RPT rows) per block
-  const int sev = (nev + RPT - 1) / RPT, sov = (nov + RPT - 1) / RPT, sew = (new_ + RPT - 1) / RPT,
-            sow = (now_ + RPT - 1) / RPT;
-  const int slots = sev + sov + sew + sow;
-  for (int t = threadIdx.x; t < slots; t += blockDim.x) {
-    int b, slot, n;
-    int boff;
-    if (t < sev) { b = 0; slot = t; n = nev; boff = (int)bo.ve; }
-    else if (t < sev + sov) { b = 1; slot = t - sev; n = nov; boff = (int)bo.vo; }
-    else if (t < sev + sov + sew) { b = 2; slot = t - sev - sov; n = new_; boff = (int)bo.we; }
-    else { b = 3; slot = t - sev - sov - sew; n = now_; boff = (int)bo.wo; }
-    // offset of block b inside a mode's 2 NZ staged entries
-    const int roff = b == 0 ? 0 : b == 1 ? nev : b == 2 ? NZ : NZ + new_;
+  const int se = (ne + RPT - 1) / RPT, slots = se + (no + RPT - 1) / RPT;  // slots (groups of RPT rows) per block
+  if (const int t = threadIdx.x; t < slots) {
+    const int b = t >= se, slot = b ? t - se : t, n = b ? no : ne;
+    const int boff = b ? odd : 0;  // offset of the block among the operator's entries,
+    const int roff = b ? ne : 0;   // and among a mode's NZ staged entries
     const int row0 = slot * RPT;
     bool live[RPT];
     int off[RPT];  // element offset of the row's current column in the group's blocks
@@ -212,7 +214,7 @@ __device__ __forceinline__ void inc_rows(cd* __restrict__ v, cd* __restrict__ g,
       const int er = rexp[roff + row];
 #pragma unroll
       for (int q = 0; q < NM; ++q) {  // S starts at sigma of mode q for this row
-        const int e = max(-120, min(120, er + s_cexp[4 * q + b] + 3));
+        const int e = max(-120, min(120, er + s_cexp[2 * q + b] + 3));
         const float sg = __int_as_float((127 + e) << 23);
         S[i][q] = pk(sg, sg);
         C[i][q] = 0ull;
@@ -293,15 +295,14 @@ __device__ __forceinline__ void inc_rows(cd* __restrict__ v, cd* __restrict__ g,
         }
     }
     columns(ma, xa, n - c0);  // the last n mod CB columns
-    cd* dst = b < 2 ? v : g;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
       if (!live[i]) continue;
       const int row = row0 + i;
-      const int j = (b == 0 || b == 2) ? 2 * row : 2 * row + 1;
+      const int j = 2 * row + b;
 #pragma unroll
       for (int q = 0; q < NM; ++q) {
-        const cd c0v = Cd[q * 2 * NZ + roff + row];
+        const cd c0v = Cd[q * NZ + roff + row];
         float Sv[2], Cv[2];
         upk(S[i][q], Sv[0], Sv[1]);
         upk(C[i][q], Cv[0], Cv[1]);
@@ -321,21 +322,12 @@ __device__ __forceinline__ void inc_rows(cd* __restrict__ v, cd* __restrict__ g,
   }
 }
 
-// block size and minimum CTAs per SM of k_inc_solve: one row per thread at
-// MV_THREADS threads (RPT = 1; blocks of more rows loop), one row per thread
-// with every row in one pass at up to MV_WIDE threads (RPT = 0, for
-// wall-normal grids of more than MV_THREADS block rows), or two rows per
-// thread at up to 256 threads (RPT = 2)
-constexpr int MV_WIDE = 416;
-template <int MCH, int RPT>
-struct IncShape {
-  static constexpr int threads = RPT == 1 ? MV_THREADS : RPT == 0 ? MV_WIDE : 256;
-  static constexpr int min_ctas = RPT == 1 ? (MCH == 2 ? 4 : 3) : 2;
-  static constexpr int rows = RPT == 0 ? 1 : RPT;  // block rows per thread
-};
-
-template <int MCH, int CB, int RPT>
-__global__ void __launch_bounds__(IncShape<MCH, RPT>::threads, IncShape<MCH, RPT>::min_ctas)
+// Threads: one row (or two) of the field each, THREADS at most, and as many
+// CTAs per SM as leave a thread 56 registers at 2 modes (five blocks of 224,
+// seven of 160) and 72 at 4 (four of 224; 64 with four of 256), 80 with two
+// rows (six blocks of 128).
+template <int MCH, int CB, int RPT, int THREADS>
+__global__ void __launch_bounds__(THREADS, RPT == 2 ? 6 : MCH == 2 && THREADS <= 224 ? 5 : 4)
     k_inc_solve(cd* __restrict__ v, cd* __restrict__ g,
                                                              const cd* __restrict__ rv, const cd* __restrict__ uh,
                                                              const cd* __restrict__ rg, const cd* __restrict__ wh,
@@ -349,70 +341,73 @@ __global__ void __launch_bounds__(IncShape<MCH, RPT>::threads, IncShape<MCH, RPT
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = d.N, NZ = d.NZ, ne = N / 2 + 1;
   const long modes = d.modes();
-  cd* Cd = reinterpret_cast<cd*>(smem_raw);                   // [MCH][2 NZ] FP64 coefficients
-  CoefHL* Cs = reinterpret_cast<CoefHL*>(Cd + MCH * 2 * NZ);  // [2 NZ][MCH] their (hi, lo) splits
-  float2* Rs = reinterpret_cast<float2*>(Cs + MCH * 2 * NZ);  // [2 NZ][MCH] folded AB2 term
+  cd* Cd = reinterpret_cast<cd*>(smem_raw);               // [MCH][NZ] FP64 coefficients
+  CoefHL* Cs = reinterpret_cast<CoefHL*>(Cd + MCH * NZ);  // [NZ][MCH] their (hi, lo) splits
+  float2* Rs = reinterpret_cast<float2*>(Cs + MCH * NZ);  // [NZ][MCH] folded AB2 term
   __shared__ int s_mode[MCH];
-  __shared__ int s_cexp[MCH * 4];  // largest |hi| per (mode, block): float bits, then its exponent
-  // work item: up to MCH modes of one k^2 group, from base
-  const int2 it = items[blockIdx.x];
-  const int grp = it.x, base = it.y;
+  __shared__ int s_cexp[MCH * 2];  // largest |hi| per (mode, block): float bits, then its exponent
+  // work item: up to MCH modes of one k^2 group, from base; one field
+  const int2 it = items[blockIdx.x >> 1];
+  const int grp = it.x, base = it.y, f = blockIdx.x & 1;
   const BlockOffsets bo = block_offsets(sl);
-  const float2* Mg = incm + (size_t)grp * sl.stride;
-  const float* Xg = incx + (size_t)grp * sl.stride;
+  const size_t first = (size_t)grp * sl.stride + (f ? bo.we : bo.ve);
+  const int odd = (int)(f ? bo.wo - bo.we : bo.vo - bo.ve);
+  const float2* Mg = incm + first;
+  const float* Xg = incx + first;
+  cd* C = f ? g : v;
+  const cd* H = f ? rg : rv;   // N^n (GL values)
+  const cd* Ho = f ? wh : uh;  // N^{n-1}
   {
     const int nm = min(MCH, group_start[grp + 1] - base);
     if (threadIdx.x < nm) s_mode[threadIdx.x] = group_modes[base + threadIdx.x];
-    if (threadIdx.x < MCH * 4) s_cexp[threadIdx.x] = 0;
+    if (threadIdx.x < MCH * 2) s_cexp[threadIdx.x] = 0;
     __syncthreads();
     // (mode, entry) loops without divisions by the run-time sizes
+    // (mode, entry) loops without divisions by the run-time sizes
     for (int q = 0; q < nm; ++q)
-    for (int i = threadIdx.x; i < 2 * NZ; i += blockDim.x) {
-      const int f = i >= NZ, k = i - f * NZ;
-      const cd x = (f == 0 ? v : g)[(size_t)k * modes + s_mode[q]];
-      const int en = f * NZ + ((k & 1) ? ne + k / 2 : k / 2);  // entry within the mode
-      Cd[q * 2 * NZ + en] = x;
-      CoefHL h;
-      bits::split(x.re, h.hr, h.lr);
-      bits::split(x.im, h.hi, h.li);
-      Cs[en * MCH + q] = h;
-      atomicMax(&s_cexp[4 * q + 2 * f + (k & 1)], __float_as_int(fmaxf(fabsf(h.hr), fabsf(h.hi))));
-    }
+      for (int k = threadIdx.x; k < NZ; k += blockDim.x) {
+        const cd x = C[(size_t)k * modes + s_mode[q]];
+        const int en = (k & 1) ? ne + k / 2 : k / 2;  // entry within the mode
+        Cd[q * NZ + en] = x;
+        CoefHL h;
+        bits::split(x.re, h.hr, h.lr);
+        bits::split(x.im, h.hi, h.li);
+        Cs[en * MCH + q] = h;
+        atomicMax(&s_cexp[2 * q + (k & 1)], __float_as_int(fmaxf(fabsf(h.hr), fabsf(h.hi))));
+      }
     // the AB2 term in FP32 (X r is an FP32 product of an O(dt) term)
     for (int q = 0; q < nm; ++q)
-    for (int i = threadIdx.x; i < 2 * ne; i += blockDim.x) {
-      const int f = i >= ne, r = i - f * ne;
-      const long m = s_mode[q];
-      const cd* H = f == 0 ? rv : rg;   // N^n (GL values)
-      const cd* Ho = f == 0 ? uh : wh;  // N^{n-1}
-      const size_t ip = (size_t)r * modes + m, iq = (size_t)(N - r) * modes + m;
-      const cd hp = H[ip], hq = H[iq], op = Ho[ip], oq = Ho[iq];
-      const float pr = c3 * bits::narrow(hp.re) - c1 * bits::narrow(op.re);
-      const float pi = c3 * bits::narrow(hp.im) - c1 * bits::narrow(op.im);
-      const float qr = c3 * bits::narrow(hq.re) - c1 * bits::narrow(oq.re);
-      const float qi = c3 * bits::narrow(hq.im) - c1 * bits::narrow(oq.im);
-      const bool wall = (f == 0) ? (r < 2) : (r < 1);
-      float2* out = Rs + (size_t)f * NZ * MCH + q;  // entry e of mode q at e MCH + q
-      out[r * MCH] = wall ? make_float2(0.f, 0.f) : make_float2(0.5f * (pr + qr), 0.5f * (pi + qi));
-      if (r < N / 2)
-        out[(ne + r) * MCH] = wall ? make_float2(0.f, 0.f) : make_float2(0.5f * (pr - qr), 0.5f * (pi - qi));
-    }
+      for (int r = threadIdx.x; r < ne; r += blockDim.x) {
+        const long m = s_mode[q];
+        const size_t ip = (size_t)r * modes + m, iq = (size_t)(N - r) * modes + m;
+        const cd hp = H[ip], hq = H[iq], op = Ho[ip], oq = Ho[iq];
+        const float pr = c3 * bits::narrow(hp.re) - c1 * bits::narrow(op.re);
+        const float pi = c3 * bits::narrow(hp.im) - c1 * bits::narrow(op.im);
+        const float qr = c3 * bits::narrow(hq.re) - c1 * bits::narrow(oq.re);
+        const float qi = c3 * bits::narrow(hq.im) - c1 * bits::narrow(oq.im);
+        const bool wall = (f == 0) ? (r < 2) : (r < 1);
+        float2* out = Rs + q;  // entry e of mode q at e MCH + q
+        out[r * MCH] = wall ? make_float2(0.f, 0.f) : make_float2(0.5f * (pr + qr), 0.5f * (pi + qi));
+        if (r < N / 2)
+          out[(ne + r) * MCH] = wall ? make_float2(0.f, 0.f) : make_float2(0.5f * (pr - qr), 0.5f * (pi - qi));
+      }
     __syncthreads();
-    if (threadIdx.x < nm * 4) {  // max < 2^e
+    if (threadIdx.x < nm * 2) {  // max < 2^e
       int e = -60;
       const float mx = __int_as_float(s_cexp[threadIdx.x]);
       if (mx > 0.f) (void)frexpf(mx, &e);
       s_cexp[threadIdx.x] = max(-60, e);
     }
     __syncthreads();
-    const signed char* rexp = rowexp + (size_t)grp * 2 * NZ;
+    const signed char* rexp = rowexp + ((size_t)grp * 2 + f) * NZ;
+    const int no = N / 2;
     switch (nm) {
-      case 1: inc_rows<1, MCH, CB, IncShape<MCH, RPT>::rows>(v, g, Mg, Xg, sl, bo, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp); break;
-      case 2: inc_rows<2, MCH, CB, IncShape<MCH, RPT>::rows>(v, g, Mg, Xg, sl, bo, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp); break;
+      case 1: inc_rows<1, MCH, CB, RPT>(C, Mg, Xg, ne, no, odd, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp); break;
+      case 2: inc_rows<2, MCH, CB, RPT>(C, Mg, Xg, ne, no, odd, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp); break;
       default:
         if constexpr (MCH >= 4) {
-          if (nm == 3) inc_rows<3, MCH, CB, IncShape<MCH, RPT>::rows>(v, g, Mg, Xg, sl, bo, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp);
-          else inc_rows<4, MCH, CB, IncShape<MCH, RPT>::rows>(v, g, Mg, Xg, sl, bo, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp);
+          if (nm == 3) inc_rows<3, MCH, CB, RPT>(C, Mg, Xg, ne, no, odd, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp);
+          else inc_rows<4, MCH, CB, RPT>(C, Mg, Xg, ne, no, odd, NZ, modes, Cd, Cs, Rs, s_mode, rexp, s_cexp);
         }
         break;
     }
@@ -718,6 +713,19 @@ __global__ void __launch_bounds__(RC_THREADS) k_inc_recover64(const cd* __restri
   }
 }
 
+using IncKernel = decltype(&k_inc_solve<4, 4, 1, 224>);
+
+template <int THREADS>
+IncKernel inc_kernel(int mch, int cb, int rpt) {
+  if (rpt == 2)
+    return mch == 2 ? (cb == 2 ? k_inc_solve<2, 2, 2, 128> : k_inc_solve<2, 3, 2, 128>)
+                    : (cb == 2 ? k_inc_solve<4, 2, 2, 128> : k_inc_solve<4, 3, 2, 128>);
+  return mch == 2 ? (cb == 2 ? k_inc_solve<2, 2, 1, THREADS>
+                             : cb == 4 ? k_inc_solve<2, 4, 1, THREADS> : k_inc_solve<2, 3, 1, THREADS>)
+                  : (cb == 2 ? k_inc_solve<4, 2, 1, THREADS>
+                             : cb == 4 ? k_inc_solve<4, 4, 1, THREADS> : k_inc_solve<4, 3, 1, THREADS>);
+}
+
 }  // namespace
 
 int setup_solver_mixed(Handle* h) {
@@ -780,6 +788,18 @@ int setup_inc_items(Handle* h) {
   return CHF_OK;
 }
 
+// Modes per CTA.  Two where a field has at most 160 rows: half the shared
+// memory and 56 registers a thread let 7 blocks of 160 threads run on an SM
+// (5 with four modes), and the runs of one group still share its operators
+// through L2.  Longer columns are closer to the memory rate, where the second
+// read of the operators costs more than the blocks in flight give.  Two
+// against four: 33 rows 12 / 15 us (32 x 33 x 32), 97 rows 160 / 158 us
+// (160 x 97 x 120), 129 rows 209 / 221 us (128 x 129 x 128), 193 rows 3245 /
+// 3089 us (384 x 193 x 384).
+int inc_modes(const Handle* h) {
+  return h->tune.inc_mch ? h->tune.inc_mch : h->d.NZ <= 160 ? 2 : 4;
+}
+
 int launch_recover(Handle* h, bool df) {
   const long modes = h->d.modes();
   auto kern = df ? k_inc_recover : k_inc_recover64;
@@ -811,21 +831,11 @@ int launch_solve_mixed(Handle* h) {
   }
   if (h->nk2 > 0) {
     const SolveLayout& sl = h->sl;
-    const int rows = sl.ne_v + sl.no_v + sl.ne_w + sl.no_w;
-    const int mch = h->tune.inc_mch == 2 ? 2 : 4, cb = h->tune.inc_cb;
-    // the wide block only where one row per thread at MV_THREADS would loop
-    const int rpt = h->tune.inc_rpt == 2 ? 2 : h->tune.inc_wide && rows > MV_THREADS ? 0 : 1;
-    auto kern = rpt == 2 ? (mch == 2 ? (cb == 2 ? k_inc_solve<2, 2, 2> : k_inc_solve<2, 3, 2>)
-                                     : (cb == 2 ? k_inc_solve<4, 2, 2> : k_inc_solve<4, 3, 2>))
-              : rpt == 0 ? (mch == 2 ? (cb == 2 ? k_inc_solve<2, 2, 0> : cb == 4 ? k_inc_solve<2, 4, 0> : k_inc_solve<2, 3, 0>)
-                                     : (cb == 2 ? k_inc_solve<4, 2, 0> : cb == 4 ? k_inc_solve<4, 4, 0> : k_inc_solve<4, 3, 0>))
-              : mch == 2 ? (cb == 2 ? k_inc_solve<2, 2, 1> : cb == 4 ? k_inc_solve<2, 4, 1> : k_inc_solve<2, 3, 1>)
-                         : (cb == 2 ? k_inc_solve<4, 2, 1> : cb == 4 ? k_inc_solve<4, 4, 1> : k_inc_solve<4, 3, 1>);
-    const int slots2 = (sl.ne_v + 1) / 2 + (sl.no_v + 1) / 2 + (sl.ne_w + 1) / 2 + (sl.no_w + 1) / 2;
-    const int threads = rpt == 1 ? MV_THREADS
-                      : rpt == 0 ? std::min(MV_WIDE, (rows + 31) / 32 * 32)
-                                 : std::min(256, (slots2 + 31) / 32 * 32);
-    const size_t smem = (sizeof(cd) + sizeof(CoefHL) + sizeof(float2)) * mch * 2 * (size_t)NZ;
+    const int mch = inc_modes(h), cb = h->tune.inc_cb, rpt = h->tune.inc_rpt;
+    const int slots = rpt == 1 ? NZ : (sl.ne_v + 1) / 2 + (sl.no_v + 1) / 2;
+    const int threads = (slots + 31) / 32 * 32;
+    auto kern = threads <= 224 ? inc_kernel<224>(mch, cb, rpt) : inc_kernel<256>(mch, cb, rpt);
+    const size_t smem = (sizeof(cd) + sizeof(CoefHL) + sizeof(float2)) * mch * (size_t)NZ;
     if (smem > 48 * 1024 &&
         !cuda_ok(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                  "k_inc_solve smem"))
@@ -833,7 +843,7 @@ int launch_solve_mixed(Handle* h) {
     prof_begin(h, K_INC_SOLVE, &ev);
     const int nitems = h->n_inc_items[mch == 4 ? 1 : 0];
     const int2* items = h->inc_items + (mch == 4 ? 0 : h->n_inc_items[1]);
-    kern<<<nitems, threads, smem, st>>>(h->f[F_V], h->f[F_OY], h->f[F_RV], h->f[F_U], h->f[F_RG],
+    kern<<<2 * nitems, threads, smem, st>>>(h->f[F_V], h->f[F_OY], h->f[F_RV], h->f[F_U], h->f[F_RG],
                                            h->f[F_W], h->incm, h->incx, h->incr_exp, h->sl, h->group_start,
                                            h->group_modes, items, d, (float)(1.5 * dt), (float)(0.5 * dt));
     prof_end(h, K_INC_SOLVE, ev);

@@ -200,8 +200,8 @@ int chf_tuning(const chf_handle* h, char* buf, int len);
  *   "inc_modes"    modes per CTA of the CHF_MIXED increment solve: 2 or 4
  *   "inc_columns"  its matrix columns per load batch: 2, 3 or 4
  *   "inc_rows"     its block rows per thread: 1 or 2 (2 with 2 or 3 columns)
- *   "inc_wide"     with one row per thread, every block row in one pass (1,
- *                  up to 416 threads) or 288-thread blocks that loop (0)
+ *   "inc_wide"     0 or 1, without effect: a block holds every row of its
+ *                  field in one pass
  *   "recover_form" arithmetic of the CHF_MIXED recovery of u, w, omega_x,
  *                  omega_z from v and omega_y: 0 FP64, 1 double-float
  *                  (about 2^-44 of the largest term), -1 the rule (double-
