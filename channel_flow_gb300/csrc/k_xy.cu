@@ -16,9 +16,15 @@
 // places (the first stage, which reads consecutive modes from global memory)
 // and lanes along the rows (all others) both spread over the banks.
 //
-// What bounds them now is the latency of their loads: at 384 x 49 x 384 the x
-// kernel issues in 44% of the cycles with the shared-memory pipe at 42% (82 to
-// 87% for the two-buffer kernels).
+// What bounds the x kernel is its instructions between barriers: at 384 x 97 x
+// 96 it issues in 59% of the cycles with the shared-memory pipe at 70%, and of
+// 109 instructions per point and line two thirds were index arithmetic, most
+// of it `slot`.  The places' slots now come from two tables in shared memory
+// (90 instructions; 293 -> 237 us there, 2264 -> 1822 us at 384 x 193 x 384,
+// 165 -> 138 us at 160 x 97 x 120).  More threads per SM at 56 registers spill
+// (2076 us at 384 x 193 x 384), and blocks sized to whole passes of the stages
+// change nothing (1822).  The y kernels have no swizzle; they run at 0.62 to
+// 0.66 of the memory rate at 384 x 193 x 384 (765 and 411 us).
 #include <algorithm>
 
 #include "chf_internal.h"
@@ -62,9 +68,13 @@ __device__ __forceinline__ C turn(C a, C w) {
 
 template <int SIGN, int R>
 __device__ __forceinline__ void twiddle(C* v, const C* __restrict__ tws, int Ns, int jm) {
+  // 32-bit byte offsets from the table's (uniform) address
+  const char* __restrict__ t = reinterpret_cast<const char*>(tws);
+  unsigned int o = (unsigned int)jm * sizeof(C);
 #pragma unroll
   for (int r = 1; r < R; ++r) {
-    v[r] = turn<SIGN>(v[r], tws[(r - 1) * Ns + jm]);
+    v[r] = turn<SIGN>(v[r], *reinterpret_cast<const C*>(t + o));
+    o += (unsigned int)Ns * sizeof(C);
   }
 }
 
@@ -174,18 +184,27 @@ __global__ void __launch_bounds__(Y_THREADS, CTAS) k_yfwd_ip(const C* __restrict
       });
 }
 
-// element of row `row` at place `at` of an x line group
+// Element of row `row` at place `at` of an x line group.  Every part of it is
+// an exclusive or of bits of `at` and `row`, so that slot(at, row) is
+// slot(at, 0) ^ row, and slot(a + b, row) is slot(a, row) ^ slot(b, 0) where a
+// and b have no bit in common.
 __device__ __forceinline__ int slot(int at, int row, int swz) {
   constexpr int RB = kRows;
   return (at >> 1) * (2 * RB) + ((at ^ (at >> swz)) & 1) * RB + (row ^ ((at >> 1) & (RB - 1)));
+}
+
+// the place of a value of slot(at, 0) (swz >= 1)
+__device__ __forceinline__ int place_of(int q, int swz) {
+  const int h = q >> 4;
+  return 2 * h + (((q >> 3) ^ (h >> (swz - 1))) & 1);
 }
 
 // x: c2r of three field pairs, the Lamb products, r2c of (H1 + i H2) and H3;
 // rows r = plane * PY + yp as in k_xprod.  ng groups of kRows rows per CTA,
 // grid ceil(nrows / (ng kRows)).  The products stand at the inverse
 // transform's places, so the forward one works at place[natural index].
-template <int X_THREADS>
-__global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __restrict__ wy, Dims d, float re_p, int ng,
+template <int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) k_xprod_ip(C* __restrict__ wy, Dims d, float re_p, int ng,
                                                         const __grid_constant__ FftPlan px,
                                                         const C* __restrict__ stab,
                                                         const unsigned short* __restrict__ tab) {
@@ -197,30 +216,39 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
   const size_t fstride = (size_t)d.MP * d.PY * KX;
   const int gl = L * RB;  // elements of one (group, pair) line set, at (g * 3 + pair) * gl
   const int nst = px.nst;
-  // the index tables in shared memory (read from the second stage on): cold
-  // misses on them would otherwise line up behind one another in every CTA
+  // the index tables in shared memory (read from the second stage on; the
+  // first computes its slots, so as not to wait for them): cold misses on them
+  // would otherwise line up behind one another in every CTA, and a slot costs
+  // seven instructions where a table read and an exclusive or cost three
   unsigned short* rev = reinterpret_cast<unsigned short*>(s + ng * 3 * gl);
-  const unsigned short* place = rev + L;
-  for (int t = tid; t < L; t += X_THREADS)
-    reinterpret_cast<unsigned int*>(rev)[t] = reinterpret_cast<const unsigned int*>(tab)[t];
+  unsigned short *at_slot = rev + L, *nat_slot = at_slot + L;  // slot(at, 0), slot(place[n], 0)
+  for (int t = tid; t < L; t += blockDim.x) {
+    rev[t] = tab[t];
+    at_slot[t] = (unsigned short)slot(t, 0, swz);
+    nat_slot[t] = (unsigned short)slot(tab[L + t], 0, swz);
+  }
   // ---- inverse, first stage: lanes along the butterflies of a row
   by_radix(px.R[0], [&]<int R>() {
     const int nr = L / R;
-    for (int t = tid; t < ng * 3 * RB * nr; t += X_THREADS) {
+    for (int t = tid; t < ng * 3 * RB * nr; t += blockDim.x) {
       const int lr = fft_div(t, px.nr_m[0], px.nr_s[0]), j = t - lr * nr;
       const int row = lr % RB, gc = lr / RB, g = gc / 3, c = gc - 3 * g;
       const long r = r0 + g * RB + row;
+      const C* __restrict__ Fr = wy + (size_t)(2 * c) * fstride + (size_t)r * KX;
+      const C* __restrict__ Gr = Fr + fstride;
+      const int kend = r < nrows ? KX : 0;
       C v[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        const int n = j + i * nr;
+        const int n = j + i * nr, k = min(n, PX - n);
         v[i] = C{(float)0, (float)0};
-        if (r < nrows && (n < KX || n > PX - KX)) {
-          const int k = n < KX ? n : PX - n;
-          const C F = wy[(size_t)(2 * c) * fstride + (size_t)r * KX + k];
-          const C G = wy[(size_t)(2 * c + 1) * fstride + (size_t)r * KX + k];
-          // F + i G, its conjugate partner, or the streamwise means (real parts)
-          v[i] = n == 0 ? C{F.re, G.re} : n < KX ? C{F.re - G.im, F.im + G.re} : C{F.re + G.im, G.re - F.im};
+        if (k < kend) {
+          const C F = Fr[k], G = Gr[k];
+          // F + i G, its conjugate partner (products by 1 or -1: exact), or
+          // the streamwise means (real parts)
+          const float u = n < KX ? 1.f : -1.f;
+          v[i] = C{__fmaf_rn(-u, G.im, F.re), __fmaf_rn(u, F.im, G.re)};
+          if (i == 0 && n == 0) v[i] = C{F.re, G.re};
         }
       }
       bfly<+1, R>(v);
@@ -229,7 +257,7 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
       for (int i = 0; i < R; ++i) lines[slot(i * nr + j, row, swz)] = v[i];
     }
   });
-  const int row = tid % RB, id = tid / RB, nid = X_THREADS / RB;
+  const int row = tid % RB, id = tid / RB, nid = blockDim.x / RB;
   // ---- inverse, middle stages, and the last one when its three butterflies
   // of a place do not fit the registers (radix above 5)
   const int rl = px.R[nst - 1];
@@ -244,12 +272,16 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
         const int hi = fft_div(bb, px.lo_m[st], px.lo_s[st]), at = hi * R * LO + bb - hi * LO;
         C* lines = s + gc * gl;
         C v[R];
+        int q[R];
 #pragma unroll
-        for (int i = 0; i < R; ++i) v[i] = lines[slot(at + i * LO, row, swz)];
+        for (int i = 0; i < R; ++i) {
+          q[i] = at_slot[at + i * LO] ^ row;
+          v[i] = lines[q[i]];
+        }
         twiddle<+1, R>(v, tws, Ns, rev[px.roff[st] + hi]);
         bfly<+1, R>(v);
 #pragma unroll
-        for (int i = 0; i < R; ++i) lines[slot(at + i * LO, row, swz)] = v[i];
+        for (int i = 0; i < R; ++i) lines[q[i]] = v[i];
       }
     });
   }
@@ -271,12 +303,15 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
         for (int b = id; b < ng * Ns; b += nid) {
           const int g = fft_div(b, px.nr_m[st], px.nr_s[st]), hi = b - g * Ns;
           const int jm = rev[px.roff[st] + hi];
+          int q[R];
+#pragma unroll
+          for (int i = 0; i < R; ++i) q[i] = at_slot[hi * R + i] ^ row;
           C v[3][R];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const C* lines = s + (g * 3 + c) * gl;
 #pragma unroll
-            for (int i = 0; i < R; ++i) v[c][i] = lines[slot(hi * R + i, row, swz)];
+            for (int i = 0; i < R; ++i) v[c][i] = lines[q[i]];
             twiddle<+1, R>(v[c], tws, Ns, jm);
             bfly<+1, R>(v[c]);
           }
@@ -285,9 +320,8 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
           for (int i = 0; i < R; ++i) {
             C z1, z2;
             products(v[0][i], v[1][i], v[2][i], z1, z2);
-            const int q = slot(hi * R + i, row, swz);
-            lines[q] = z1;
-            lines[gl + q] = z2;
+            lines[q[i]] = z1;
+            lines[gl + q[i]] = z2;
           }
         }
       }
@@ -295,7 +329,7 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
   } else {
     for (int b = id; b < ng * L; b += nid) {
       const int g = b / L;
-      C* lines = s + g * 3 * gl + slot(b - g * L, row, swz);
+      C* lines = s + g * 3 * gl + (at_slot[b - g * L] ^ row);
       C z1, z2;
       products(lines[0], lines[gl], lines[2 * gl], z1, z2);
       lines[0] = z1;
@@ -316,7 +350,7 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
         int q[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-          q[i] = slot(place[at + i * LO], row, swz);
+          q[i] = nat_slot[at + i * LO] ^ row;
           v[i] = lines[q[i]];
         }
         if (st > 0) twiddle<-1, R>(v, tws, Ns, rev[px.roff[st] + hi]);
@@ -335,22 +369,23 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
     wy[2 * fstride + (size_t)r * KX + k] = H3;
   };
   if (fuse) {
-    // butterflies jm and Ns - jm hold each other's Z[-k]
+    // butterflies jm and Ns - jm hold each other's Z[-k]; 0 and (Ns even)
+    // Ns / 2 hold their own and share a task
     by_radix(rl, [&]<int R>() {
       if constexpr (R <= 5) {
-        const int st = nst - 1, Ns = px.Ns[st], half = Ns / 2 + 1;
+        const int st = nst - 1, Ns = px.Ns[st], half = (Ns + 1) / 2;
         const C* __restrict__ tws = stab + px.twoff[st];
         for (int b = id; b < ng * half; b += nid) {
-          const int g = b / half, jm = b - g * half, jn = jm == 0 ? 0 : Ns - jm;
+          const int g = b / half, jm = b - g * half, jn = jm > 0 ? Ns - jm : Ns % 2 ? 0 : Ns / 2;
           const long r = r0 + g * RB + row;
           C z[2][R], h[2][R];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int j = e ? jn : jm, at = place[j];
+            const int j = e ? jn : jm, at = place_of(nat_slot[j], swz);
             const C* lines = s + g * 3 * gl;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-              const int q = slot(place[at + i], row, swz);
+              const int q = nat_slot[at + i] ^ row;
               z[e][i] = lines[q];
               h[e][i] = lines[gl + q];
             }
@@ -367,7 +402,7 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
             for (int i = 0; i < R; ++i) {
               const int k = (e ? jn : jm) + i * Ns;
               if (k >= KX) continue;
-              const C B = jm == 0 ? z[0][(R - i) % R] : z[1 - e][R - 1 - i];
+              const C B = jm > 0 ? z[1 - e][R - 1 - i] : e ? z[1][R - 1 - i] : z[0][(R - i) % R];
               emit(r, k, z[e][i], B, h[e][i]);
             }
           }
@@ -380,8 +415,8 @@ __global__ void __launch_bounds__(X_THREADS, 1024 / X_THREADS) k_xprod_ip(C* __r
       const long r = r0 + g * RB + row;
       if (r >= nrows) continue;
       const C* lines = s + g * 3 * gl;
-      const int q = slot(place[place[k]], row, swz);
-      const int qn = slot(place[place[k == 0 ? 0 : PX - k]], row, swz);
+      const int q = nat_slot[place_of(nat_slot[k], swz)] ^ row;
+      const int qn = nat_slot[place_of(nat_slot[k == 0 ? 0 : PX - k], swz)] ^ row;
       emit(r, k, lines[q], lines[qn], lines[gl + q]);
     }
   }
@@ -407,11 +442,13 @@ int pack(size_t set_bytes, int set_tasks, long sets, int threads, long ctas) {
   return n;
 }
 
+constexpr size_t kSmSmem = 228 * 1024;  // shared memory of an SM; a CTA takes 1 KB more than it asks for
+
 }  // namespace
 
 // Whether the in-place kernels serve these lines: they hold whole tiles of
-// lines per CTA (y 128 L bytes, x 196 L bytes).
-bool xy_in_place(const Dims& d) { return 128 * (size_t)d.PY <= kMaxSmem && 196 * (size_t)d.PX <= kMaxSmem; }
+// lines per CTA (y 128 L bytes, x 198 L bytes).
+bool xy_in_place(const Dims& d) { return 128 * (size_t)d.PY <= kMaxSmem && 198 * (size_t)d.PX <= kMaxSmem; }
 
 int launch_y_in_place(Handle* h, cf* wz, cf* wy, const FftPlan& py, const cf* stab, const unsigned short* rev,
                       bool inverse) {
@@ -439,15 +476,14 @@ int launch_y_in_place(Handle* h, cf* wz, cf* wy, const FftPlan& py, const cf* st
 int launch_x_in_place(Handle* h, cf* wy, const FftPlan& px, const cf* stab, const unsigned short* tab) {
   const Dims d = fft_view(h->d);
   const long nrows = (long)d.MP * d.PY;
-  const size_t set = 192 * (size_t)d.PX;
+  const size_t set = 192 * (size_t)d.PX, tables = 6 * (size_t)d.PX;
   // 1024 threads per SM either way: four small CTAs where their lines fit
-  const size_t tables = 4 * (size_t)d.PX;
-  const bool small = 4 * (set + tables) <= kMaxSmem;
+  const bool small = 4 * (set + tables + 1024) <= kSmSmem;
   const int threads = small ? 256 : 512;
   const int ng = pack(set, 3 * kRows * (px.L / px.R[0]), (nrows + kRows - 1) / kRows, threads,
                       nrows / kRows / h->num_sms);
   const long per = (long)ng * kRows;
-  auto kern = small ? k_xprod_ip<256> : k_xprod_ip<512>;
+  auto kern = small ? k_xprod_ip<256, 4> : k_xprod_ip<512, 2>;
   cudaEvent_t ev;
   if (!set_smem(h, kern, ng * set + tables)) return CHF_E_CUDA;
   prof_begin(h, K_XPROD, &ev);
