@@ -217,6 +217,8 @@ struct Handle {
   // matrices' digit fragments followed by the tables they come from
   TfPlan tf_z1{}, tf_gl{}, tf_z2{}, tf_yi{}, tf_yf{}, tf_xi{}, tf_xf{};
   void* tf_image = nullptr;
+  TfPlan tf_oz{}, tf_oy{}, tf_ox{};  // unpadded (setup_tf_out)
+  void* tf_out_image = nullptr;
   void* scratch = nullptr;  // reduction scratch (diagnostics)
   void* stats_buf = nullptr;  // chf_statistics: GL values of u, v, w + plane sums (first call)
   void* pres_buf = nullptr;   // chf_pressure: Lamb coefficients, right-hand sides, P (first call)
@@ -367,6 +369,10 @@ int launch_tf_c2v(Handle* h);
 int launch_tf_xy(Handle* h);
 int launch_tf_v2c(Handle* h, cd* const* hc);
 int launch_tf_curl(Handle* h);
+bool tf_phys(const Dims& d);
+int setup_tf_out(Handle* h);
+int launch_tf_gl(Handle* h, const cd* const* in, cd* const* out, int n);
+int launch_tf_plane(Handle* h, cd* const* f, int n);
 int launch_meanfix(Handle* h);  // k_mixed.cu
 // in-place x / y transforms of FP32 lines (k_xy.cu)
 bool xy_in_place(const Dims& d);

@@ -27,6 +27,10 @@
 // The reference moves the data between ranks with its pencil transposes in
 // between; on one GPU each pass walks the contiguous index of its layout
 // instead.
+//
+// u, v, w of the state (the CFL numbers and the velocity dump) go through the
+// digit products of k_dft64.cu instead where the lines are short enough
+// (velocity_to_physical): the FP64 pipe bounds the FFT passes.
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -320,12 +324,23 @@ cd* phys_field(Handle* h, int i) {
   return reinterpret_cast<cd*>(static_cast<char*>(h->phys_buf) + (size_t)i * sizeof(cd) * h->d.field_elems());
 }
 
-// u, v, w of the resident state on the physical grid in phys_field 0, 1, 2
+// u, v, w of the resident state on the physical grid in phys_field 0, 1, 2.
+// Lines of at most 384 points: exact digit products on the tensor cores
+// (k_dft64.cu), three launches for the three fields; longer ones, where the
+// dense product has no advantage left, the FFT passes above.  A whole CFL call,
+// FFTs / digits: 32^3 99 / 48 us, 96 x 72 x 80 387 / 144, 128^3 990 / 370,
+// 320 x 192 x 96 2855 / 1427, 256 x 256 x 128 3720 / 1808.
 int velocity_to_physical(Handle* h) {
   int rc = ensure_phys(h);
   if (rc != CHF_OK) return rc;
   const size_t fb = sizeof(cd) * h->d.field_elems();
   const int src[3] = {F_U, F_V, F_W};
+  if (tf_phys(h->d)) {
+    const cd* in[3] = {h->f[F_U], h->f[F_V], h->f[F_W]};
+    cd* out[3] = {phys_field(h, 0), phys_field(h, 1), phys_field(h, 2)};
+    if ((rc = setup_tf_out(h)) != CHF_OK || (rc = launch_tf_gl(h, in, out, 3)) != CHF_OK) return rc;
+    return launch_tf_plane(h, out, 3);
+  }
   for (int i = 0; i < 3; ++i) {
     if (!cuda_ok(h, cudaMemcpyAsync(phys_field(h, i), h->f[src[i]], fb, cudaMemcpyDeviceToDevice, h->stream),
                  "physical copy"))

@@ -12,7 +12,9 @@
 //   <f'g'>(z_k) = sum over modes (kx, ky) != (0, 0) of w_kx Re(f^(z_k) conj(g^(z_k))),
 // with w_kx = 1 for kx = 0 and 2 for kx > 0 (the half spectrum in x), and
 // <f>(z_k) = Re f^_{00}(z_k).  The only transform is Chebyshev coefficients
-// -> Gauss-Lobatto values, one 2N-point DFT per (field, mode) line.
+// -> Gauss-Lobatto values, as exact digit products (k_dft64.cu).  A whole call
+// at 128^3 takes 202 us, with the FFTs of these lines it took 466; at 32^3
+// 47 / 58 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -26,48 +28,8 @@ struct chf_handle : public Handle {};
 
 namespace {
 
-constexpr int ST_LINES = 4;    // (field, mode) lines per CTA
 constexpr int ST_THREADS = 256;
 constexpr int NSTAT = 10;      // per plane: <u>,<v>,<w>, uu,vv,ww, uv,uw,vw, energy density
-
-// GL values of u, v, w (fields 0..2) for every mode: out[f][k][mode]
-template <int MB2>
-__global__ void __launch_bounds__(ST_THREADS) k_stat_gl(const cd* __restrict__ u, const cd* __restrict__ v,
-                                                       const cd* __restrict__ w, cd* __restrict__ out, Dims d,
-                                                       const __grid_constant__ FftPlan pz2,
-                                                       const cd* __restrict__ tw2) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cd* s = reinterpret_cast<cd*>(smem_raw);
-  const int N = d.N, NZ = d.NZ, L2 = 2 * N;
-  const long modes = d.modes(), lines = 3 * modes;
-  const long l0 = (long)blockIdx.x * ST_LINES;
-  for (int t = threadIdx.x; t < ST_LINES * NZ; t += blockDim.x) {
-    const int l = t / NZ, n = t % NZ;
-    const long line = l0 + l;
-    cd c{0.0, 0.0};
-    if (line < lines) {
-      const int f = (int)(line / modes);
-      const long m = line % modes;
-      const cd* src = f == 0 ? u : f == 1 ? v : w;
-      c = src[(size_t)n * modes + m];
-    }
-    // even extension with doubled end coefficients: 0.5 DFT = values at z_k
-    const double dbl = (n == 0 || n == N) ? 2.0 : 1.0;
-    s[l * L2 + n] = cd{dbl * c.re, dbl * c.im};
-    if (n > 0 && n < N) s[l * L2 + L2 - n] = c;
-  }
-  __syncthreads();
-  smem_fft<double, -1, MB2>(s, ST_LINES, L2, pz2, tw2);
-  for (int t = threadIdx.x; t < ST_LINES * NZ; t += blockDim.x) {
-    const int l = t / NZ, k = t % NZ;
-    const long line = l0 + l;
-    if (line >= lines) continue;
-    const int f = (int)(line / modes);
-    const long m = line % modes;
-    const cd x = s[l * L2 + k];
-    out[((size_t)f * NZ + k) * modes + m] = cd{0.5 * x.re, 0.5 * x.im};
-  }
-}
 
 // one CTA per plane k: means, covariances and sum_modes w (|u|^2+|v|^2+|w|^2)
 __global__ void __launch_bounds__(ST_THREADS) k_stat_sum(const cd* __restrict__ gl, Dims d, double* __restrict__ out) {
@@ -124,27 +86,17 @@ extern "C" int chf_statistics(chf_handle* h, double* profiles, chf_stats* out) {
   if (!cuda_ok(h, cudaSetDevice(h->device), "cudaSetDevice")) return CHF_E_CUDA;
   const Dims& d = h->d;
   const int N = d.N, NZ = d.NZ;
-  const long modes = d.modes();
-  const size_t gl_elems = (size_t)3 * NZ * modes;
+  const size_t gl_elems = (size_t)3 * NZ * d.modes();
   if (!h->stats_buf) {  // first call: GL values of three fields + plane sums
     const size_t bytes = sizeof(cd) * gl_elems + sizeof(double) * (size_t)NZ * NSTAT;
     if (!cuda_ok(h, cudaMalloc(&h->stats_buf, bytes), "statistics buffer")) return CHF_E_NOMEM;
   }
   cd* gl = static_cast<cd*>(h->stats_buf);
   double* sums = reinterpret_cast<double*>(gl + gl_elems);
-  const int mb2 = fft_fits(ST_LINES, 2 * N, ST_THREADS, 2) ? 2 : 4;
-  if (!fft_fits(ST_LINES, 2 * N, ST_THREADS, mb2)) {
-    h->err = "chf_statistics: nnz too large";
-    return CHF_E_INVALID;
-  }
-  const size_t smem = sizeof(cd) * ST_LINES * 2 * N;
-  auto kern = mb2 == 2 ? k_stat_gl<2> : k_stat_gl<4>;
-  if (smem > 48 * 1024 &&
-      !cuda_ok(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "stats smem"))
-    return CHF_E_CUDA;
-  const long lines = 3 * modes;
-  kern<<<(unsigned)((lines + ST_LINES - 1) / ST_LINES), ST_THREADS, smem, h->stream>>>(
-      h->f[F_U], h->f[F_V], h->f[F_W], gl, d, h->pz2, h->tw_z2);
+  const cd* in[3] = {h->f[F_U], h->f[F_V], h->f[F_W]};
+  cd* val[3] = {gl, gl + gl_elems / 3, gl + 2 * (gl_elems / 3)};
+  int rc;
+  if ((rc = setup_tf_out(h)) != CHF_OK || (rc = launch_tf_gl(h, in, val, 3)) != CHF_OK) return rc;
   k_stat_sum<<<NZ, ST_THREADS, 0, h->stream>>>(gl, d, sums);
   if (!cuda_ok(h, cudaGetLastError(), "statistics kernels")) return CHF_E_CUDA;
   std::vector<double> S((size_t)NZ * NSTAT), au0(2 * (size_t)NZ);

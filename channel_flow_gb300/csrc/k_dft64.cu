@@ -480,18 +480,19 @@ TfShape tf_shape(int L, int ke, int ko, int ne, int no) {
 
 
 template <int MODE>
-int launch_tf(Handle* h, const TfPlan& p, const double* const* in, double* const* out, int nfields, long lines, int kid) {
+int launch_tf(Handle* h, const Dims& d, const TfPlan& p, const double* const* in, double* const* out, int nfields,
+              long lines, int kid) {  // kid < 0: not one of a step's kernels
   TfArgs a{};
   for (int i = 0; i < nfields; ++i) {
     a.in[i] = in[i];
     a.out[i] = out[i];
   }
   a.nfields = nfields;
-  a.scale = MODE == TF_YFWD ? 1.0 / ((double)h->d.PX * (double)h->d.PY) : MODE == TF_Z2 ? 1.0 / (double)h->d.MZ : 1.0;
+  a.scale = MODE == TF_YFWD ? 1.0 / ((double)d.PX * (double)d.PY) : MODE == TF_Z2 ? 1.0 / (double)d.MZ : 1.0;
   a.mat = static_cast<const uint4*>(p.mat);
   a.s = p.s;
   a.lines = lines;
-  a.d = h->d;
+  a.d = d;
   const size_t smem = tf_smem(p.s);
   if (!cuda_ok(h, cudaFuncSetAttribute(k_tf<MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared),
@@ -500,9 +501,9 @@ int launch_tf(Handle* h, const TfPlan& p, const double* const* in, double* const
     return CHF_E_CUDA;
   const int per = MODE == TF_YINV || MODE == TF_YFWD ? TF_LINES / 2 : TF_LINES;
   cudaEvent_t ev;
-  prof_begin(h, kid, &ev);
+  if (kid >= 0) prof_begin(h, kid, &ev);
   k_tf<MODE><<<(unsigned)((lines + per - 1) / per * nfields), TF_THREADS, smem, h->stream>>>(a);
-  prof_end(h, kid, ev);
+  if (kid >= 0) prof_end(h, kid, ev);
   return cuda_ok(h, cudaGetLastError(), "k_tf") ? CHF_OK : CHF_E_CUDA;
 }
 
@@ -567,51 +568,40 @@ constexpr int kTfMaxZ = 512, kTfMaxXY = 384;
 bool tf_z(const Dims& d) { return d.nch == 1 && d.MZ <= kTfMaxZ; }
 bool tf_xy(const Dims& d) { return d.nch == 1 && d.PX <= kTfMaxXY && d.PY <= kTfMaxXY; }
 
-int setup_tf(Handle* h) {
-  const Dims& d = h->d;
-  if (!(tf_z(d) || tf_xy(d)) || h->tf_image) return CHF_OK;
-  struct Item {
-    TfPlan* p;
-    int mode, period;
-  };
-  const int M = d.MZ, N = d.N;
-  h->tf_z1.s = tf_shape(M, N / 2 + 1, N / 2, M / 2 + 1, (M + 1) / 2);
-  h->tf_gl.s = tf_shape(N, N / 2 + 1, N / 2, N / 2 + 1, N / 2);
-  h->tf_z2.s = tf_shape(M, M / 2 + 1, (M + 1) / 2, N / 2 + 1, N / 2);
-  h->tf_yi.s = tf_shape(d.PY, d.NYQ, d.NYQ, d.PY / 2 + 1, d.PY / 2);
-  h->tf_yf.s = tf_shape(d.PY, d.PY / 2 + 1, d.PY / 2, d.NYQ + 1, d.NYQ + 1);
-  h->tf_xi.s = tf_shape(d.PX, d.KX, d.KX, d.PX / 2 + 1, d.PX / 2);
-  h->tf_xf.s = tf_shape(d.PX, d.PX / 2 + 1, d.PX / 2, d.KX, d.KX);
-  const Item all[] = {{&h->tf_z1, TF_Z, 2 * M},
-                      {&h->tf_gl, TF_Z, 2 * N},
-                      {&h->tf_z2, TF_Z2, 2 * M},
-                      {&h->tf_yi, TF_YINV, d.PY},
-                      {&h->tf_yf, TF_YFWD, d.PY},
-                      {&h->tf_xi, TF_XINV, d.PX},
-                      {&h->tf_xf, TF_XFWD, d.PX}};
-  const std::vector<Item> items(all + (tf_z(d) ? 0 : 3), all + (tf_xy(d) ? 7 : 3));
+// the unpadded lines of the physical velocity: the same lengths (chf_phys.cu has the figures)
+bool tf_phys(const Dims& d) { return d.nch == 1 && d.nnx <= kTfMaxXY && d.nny <= kTfMaxXY; }
+
+namespace {
+
+struct TfItem {
+  TfPlan* p;
+  int mode, period;
+};
+
+// the digit matrices of the items' plans, in one allocation *image
+int build_tf(Handle* h, const std::vector<TfItem>& items, void** image) {
   size_t vecs = 0, entries = 0;
-  for (const Item& it : items) {
+  for (const TfItem& it : items) {
     vecs += tf_mat_vecs(it.p->s);
     entries += 2 * (size_t)it.period;
   }
   std::vector<long long> host;
   host.reserve(entries);
-  for (const Item& it : items) {
+  for (const TfItem& it : items) {
     it.p->s.f = it.mode == TF_XINV || it.mode == TF_Z2 ? 1 : 0;
     std::vector<long long> cs, sn;
     trig_table(it.period, ldexpl(1.0L, 62 - it.p->s.f), cs, sn);
     host.insert(host.end(), cs.begin(), cs.end());
     host.insert(host.end(), sn.begin(), sn.end());
   }
-  if (!cuda_ok(h, cudaMalloc(&h->tf_image, sizeof(uint4) * vecs + sizeof(long long) * entries), "transform digits"))
+  if (!cuda_ok(h, cudaMalloc(image, sizeof(uint4) * vecs + sizeof(long long) * entries), "transform digits"))
     return CHF_E_NOMEM;
-  uint4* mat = static_cast<uint4*>(h->tf_image);
+  uint4* mat = static_cast<uint4*>(*image);
   const long long* tab = reinterpret_cast<const long long*>(mat + vecs);
   if (!cuda_ok(h, cudaMemcpyAsync((void*)tab, host.data(), sizeof(long long) * entries, cudaMemcpyHostToDevice, h->stream),
                "transform tables"))
     return CHF_E_CUDA;
-  for (const Item& it : items) {
+  for (const TfItem& it : items) {
     const TfShape& s = it.p->s;
     it.p->mat = mat;
     const int blocks = (int)((tf_mat_vecs(s) / 128 + 3) / 4);
@@ -629,6 +619,69 @@ int setup_tf(Handle* h) {
   return CHF_OK;
 }
 
+}  // namespace
+
+int setup_tf(Handle* h) {
+  const Dims& d = h->d;
+  if (!(tf_z(d) || tf_xy(d)) || h->tf_image) return CHF_OK;
+  const int M = d.MZ, N = d.N;
+  h->tf_z1.s = tf_shape(M, N / 2 + 1, N / 2, M / 2 + 1, (M + 1) / 2);
+  h->tf_gl.s = tf_shape(N, N / 2 + 1, N / 2, N / 2 + 1, N / 2);
+  h->tf_z2.s = tf_shape(M, M / 2 + 1, (M + 1) / 2, N / 2 + 1, N / 2);
+  h->tf_yi.s = tf_shape(d.PY, d.NYQ, d.NYQ, d.PY / 2 + 1, d.PY / 2);
+  h->tf_yf.s = tf_shape(d.PY, d.PY / 2 + 1, d.PY / 2, d.NYQ + 1, d.NYQ + 1);
+  h->tf_xi.s = tf_shape(d.PX, d.KX, d.KX, d.PX / 2 + 1, d.PX / 2);
+  h->tf_xf.s = tf_shape(d.PX, d.PX / 2 + 1, d.PX / 2, d.KX, d.KX);
+  const TfItem all[] = {{&h->tf_z1, TF_Z, 2 * M},
+                        {&h->tf_gl, TF_Z, 2 * N},
+                        {&h->tf_z2, TF_Z2, 2 * M},
+                        {&h->tf_yi, TF_YINV, d.PY},
+                        {&h->tf_yf, TF_YFWD, d.PY},
+                        {&h->tf_xi, TF_XINV, d.PX},
+                        {&h->tf_xf, TF_XFWD, d.PX}};
+  return build_tf(h, std::vector<TfItem>(all + (tf_z(d) ? 0 : 3), all + (tf_xy(d) ? 7 : 3)), &h->tf_image);
+}
+
+// The unpadded transforms of the statistics and the physical velocity: values
+// at the Gauss-Lobatto points, and (tf_phys) on the nnx x nny points of a plane.
+int setup_tf_out(Handle* h) {
+  if (h->tf_out_image) return CHF_OK;
+  const Dims& d = h->d;
+  h->tf_oz.s = tf_shape(d.N, d.N / 2 + 1, d.N / 2, d.N / 2 + 1, d.N / 2);
+  std::vector<TfItem> items{{&h->tf_oz, TF_Z, 2 * d.N}};
+  if (tf_phys(d)) {
+    h->tf_oy.s = tf_shape(d.nny, d.NYQ, d.NYQ, d.nny / 2 + 1, d.nny / 2);
+    h->tf_ox.s = tf_shape(d.nnx, d.KX, d.KX, d.nnx / 2 + 1, d.nnx / 2);
+    items.push_back({&h->tf_oy, TF_YINV, d.nny});
+    items.push_back({&h->tf_ox, TF_XINV, d.nnx});
+  }
+  return build_tf(h, items, &h->tf_out_image);
+}
+
+// coefficients -> values at the Gauss-Lobatto points, n fields
+int launch_tf_gl(Handle* h, const cd* const* in, cd* const* out, int n) {
+  const double* i[6];
+  double* o[6];
+  for (int f = 0; f < n; ++f) {
+    i[f] = reinterpret_cast<const double*>(in[f]);
+    o[f] = reinterpret_cast<double*>(out[f]);
+  }
+  return launch_tf<TF_Z>(h, h->d, h->tf_oz, i, o, n, 2 * h->d.modes(), -1);
+}
+
+// Gauss-Lobatto values -> the physical nnx x nny planes, each field in place:
+// a CTA has its lines in shared memory before it writes the first of them, and
+// the unpadded lines take the place they had.
+int launch_tf_plane(Handle* h, cd* const* f, int n) {
+  Dims d = h->d;
+  d.PX = d.nnx;
+  d.PY = d.nny;
+  double* x[6];
+  for (int i = 0; i < n; ++i) x[i] = reinterpret_cast<double*>(f[i]);
+  const int rc = launch_tf<TF_YINV>(h, d, h->tf_oy, x, x, n, (long)d.NZ * d.KX, -1);
+  return rc != CHF_OK ? rc : launch_tf<TF_XINV>(h, d, h->tf_ox, x, x, n, (long)d.NZ * d.nny, -1);
+}
+
 size_t tf_phys_elems(const Dims& d) { return tf_xy(d) ? (size_t)6 * d.MP * d.PY * d.PX : 0; }
 
 // the six fields' values on the product grid: state -> wz
@@ -641,7 +694,7 @@ int launch_tf_c2v(Handle* h) {
     in[i] = reinterpret_cast<const double*>(h->f[order[i]]);
     out[i] = reinterpret_cast<double*>(h->wz + i * zf);
   }
-  return launch_tf<TF_Z>(h, h->tf_z1, in, out, 6, 2 * h->d.modes(), K_ZC2V);
+  return launch_tf<TF_Z>(h, h->d, h->tf_z1, in, out, 6, 2 * h->d.modes(), K_ZC2V);
 }
 
 // y and x inverse, products, x and y forward: wz -> wy -> wp -> wy -> wz (three components)
@@ -656,16 +709,16 @@ int launch_tf_xy(Handle* h) {
   }
   const long ylines = (long)d.MP * d.KX, rows = (long)d.MP * d.PY;
   int rc;
-  if ((rc = launch_tf<TF_YINV>(h, h->tf_yi, z, y, 6, ylines, K_YINV)) != CHF_OK ||
-      (rc = launch_tf<TF_XINV>(h, h->tf_xi, y, x, 6, rows, K_XINV)) != CHF_OK)
+  if ((rc = launch_tf<TF_YINV>(h, h->d, h->tf_yi, z, y, 6, ylines, K_YINV)) != CHF_OK ||
+      (rc = launch_tf<TF_XINV>(h, h->d, h->tf_xi, y, x, 6, rows, K_XINV)) != CHF_OK)
     return rc;
   cudaEvent_t ev;
   prof_begin(h, K_LAMB64, &ev);
   k_lamb64<<<(unsigned)((xf / 2 + 255) / 256), 256, 0, h->stream>>>(h->wp, xf, h->cfg.re_p);
   prof_end(h, K_LAMB64, ev);
   if (!cuda_ok(h, cudaGetLastError(), "k_lamb64")) return CHF_E_CUDA;
-  if ((rc = launch_tf<TF_XFWD>(h, h->tf_xf, x, y, 3, rows, K_XPROD)) != CHF_OK) return rc;
-  return launch_tf<TF_YFWD>(h, h->tf_yf, y, z, 3, ylines, K_YFWD);
+  if ((rc = launch_tf<TF_XFWD>(h, h->d, h->tf_xf, x, y, 3, rows, K_XPROD)) != CHF_OK) return rc;
+  return launch_tf<TF_YFWD>(h, h->d, h->tf_yf, y, z, 3, ylines, K_YFWD);
 }
 
 // the Lamb vector's coefficients from its three components on the product
@@ -678,7 +731,7 @@ int launch_tf_v2c(Handle* h, cd* const* hc) {
     in[i] = reinterpret_cast<const double*>(h->wz + i * zf);
     out[i] = reinterpret_cast<double*>(hc[i]);
   }
-  return launch_tf<TF_Z2>(h, h->tf_z2, in, out, 3, 2 * h->d.modes(), K_ZFWD);
+  return launch_tf<TF_Z2>(h, h->d, h->tf_z2, in, out, 3, 2 * h->d.modes(), K_ZFWD);
 }
 
 // values of the Lamb vector's components on the product grid (wz) -> histories
@@ -703,7 +756,7 @@ int launch_tf_curl(Handle* h) {
   if (!cuda_ok(h, cudaGetLastError(), "k_curl64")) return CHF_E_CUDA;
   const double* in[6] = {hv, hg};
   double* out[6] = {reinterpret_cast<double*>(h->f[F_U]), reinterpret_cast<double*>(h->f[F_W])};
-  if ((rc = launch_tf<TF_Z>(h, h->tf_gl, in, out, 2, cols, K_GL64)) != CHF_OK) return rc;
+  if ((rc = launch_tf<TF_Z>(h, h->d, h->tf_gl, in, out, 2, cols, K_GL64)) != CHF_OK) return rc;
   return launch_meanfix(h);
 }
 

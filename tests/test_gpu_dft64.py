@@ -124,3 +124,24 @@ def test_laminar_flow_stays_laminar(chflow_lib, nnx, nny, nnz):
         assert not np.any(out[k]), k
     for k in ("omegaxnp1", "omegaznp1"):  # H1, H3 are left there; the mean mode's H1 holds -re_p
         assert not np.any(out[k][:, 1:, :]) and not np.any(out[k][:, 0, 2:]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nnx,nny,nnz", [(4, 4, 4), (20, 36, 10), (60, 100, 32), (384, 12, 8), (12, 384, 250), (96, 64, 128)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_physical_velocity_equals_the_transform(chflow_lib, nnx, nny, nnz, precision):
+    """The unpadded digit products (physical velocity, CFL numbers) against the
+    FFT passes of chf_transform, which take one field at a time.  An FFT's
+    rounding is at most a few ulp a stage of the line's norm, three lines in
+    turn: 1e-12 of the largest value covers 30 stages."""
+    cfg = config.small(nnx=nnx, nny=nny, nnz=nnz, aphi=1.0, beta=0.5, dt=1e-4, re=180.0, re_p=1.0)
+    st = fields.reference_like_state(cfg, seed=2, epsilon=0.3, noise=0.02, gamma=3.0)
+    with Channel(cfg, precision=precision) as g:
+        g.upload_state(st)
+        got = g.physical_velocity()
+        ref = [g.transform(1, st[k]) for k in ("unp1", "wnp1", "vnp1")]
+        cfl = g.cfl()
+    for a, b in zip(got, ref):
+        assert np.abs(a - b.reshape(a.shape)).max() <= 1e-12 * np.abs(b).max()
+    umax = np.abs(ref[0]).max() * cfg.dt / (cfg.aphi * 2 * np.pi / nnx)
+    assert abs(cfl["cfl_x"] - umax) <= 1e-12 * umax

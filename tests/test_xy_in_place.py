@@ -51,7 +51,8 @@ def test_place_tables_give_the_dft(radices):
 # nnx, nny, nnz: PX and PY = 6..576 (radices 3.2 | 8.9 | 16.3 | 16.9 | 9.4.5 | 16.9.4 ...); the
 # second and third rows have planes enough for the in-place x kernel (32 rows per SM)
 GRIDS = [(4, 4, 4), (32, 32, 16), (20, 72, 10), (160, 120, 6),
-         (12, 384, 16), (48, 96, 24), (96, 72, 32), (160, 120, 30), (384, 64, 54), (20, 60, 60), (576, 120, 20)]
+         (12, 384, 16), (48, 96, 24), (96, 72, 32), (160, 120, 30), (384, 64, 54), (20, 60, 60), (576, 120, 20),
+         (24, 96, 32), (120, 64, 32)]  # the last two: an odd number of last butterflies
 
 
 @pytest.mark.gpu
