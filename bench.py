@@ -206,6 +206,49 @@ def kernel_work(cfg, zpad=0, precision="fp64", recover_df=False):
     return w
 
 
+def digit_work(cfg, zpad, ran):
+    """(bytes, flops, pipe) of the CHF_FP64 kernels that run as exact digit
+    products (csrc/k_dft64.cu, k_solve64.cu) among the names in `ran`: 36
+    FP16 products make one FP64 product, so their bound is the tensor pipe;
+    the products and recurrences between them count FP64 operations."""
+    import numpy as np
+    from channel_flow_gb300.fields import wavenumbers
+    N = cfg.nnz
+    NZ, KX, KY = N + 1, cfg.nnx // 2, cfg.nny
+    PX, PY, MZ = 3 * cfg.nnx // 2, 3 * cfg.nny // 2, zpad or 2 * N
+    MP, modes, c = MZ + 1, KX * KY, 16
+    ne, no = N // 2 + 1, N // 2
+    digit = 36 * 2.0  # flops per FP64 product
+
+    def halves(lines, ke, nev, ko, nod):  # an even and an odd half per real line
+        return digit * lines * (ke * nev + ko * nod)
+
+    me, mo = MZ // 2 + 1, (MZ + 1) // 2
+    w = {}
+    if "k_zfwd" in ran:
+        w["k_zc2v"] = (6 * (NZ + MP) * modes * c, halves(12 * modes, ne, me, no, mo), "tensor")
+        w["k_zfwd"] = (3 * (NZ + MP) * modes * c, halves(6 * modes, me, ne, mo, no), "tensor")
+        w["k_zgl"] = (4 * NZ * modes * c, halves(4 * modes, ne, ne, no, no), "tensor")
+        w["k_curl"] = (5 * NZ * modes * c, modes * NZ * 2 * 10, "fp64")
+    if "k_xinv" in ran:
+        ylines, rows, xb = 2 * MP * KX, MP * PY, MP * PY * KX * c
+        w["k_yinv"] = (6 * (MP * modes * c + xb), halves(6 * ylines, KY // 2, PY // 2 + 1, KY // 2, PY // 2), "tensor")
+        w["k_yfwd"] = (3 * (MP * modes * c + xb), halves(3 * ylines, PY // 2 + 1, KY // 2 + 1, PY // 2, KY // 2 + 1),
+                       "tensor")
+        w["k_xinv"] = (6 * (xb + rows * PX * 8), halves(6 * rows, KX, PX // 2 + 1, KX, PX // 2), "tensor")
+        w["k_xprod"] = (3 * (xb + rows * PX * 8), halves(3 * rows, PX // 2 + 1, KX, PX // 2, KX), "tensor")
+        w["k_lamb"] = (9 * rows * PX * 8, 10.0 * rows * PX, "fp64")
+    if "k_inc_recover" in ran:  # the increment form: M and X, eight digit bytes an entry
+        ia, ib = wavenumbers(cfg)
+        k2 = (ia[None, :] ** 2 + ib[:, None] ** 2)
+        k2[KY // 2, :] = 0.0
+        nk2, nsolve = len(np.unique(k2[k2 != 0.0])), int((k2 != 0.0).sum())
+        stride = 2 * (ne * ne + no * no)
+        w["k_solve"] = (nk2 * stride * 16 + 8 * NZ * modes * c, digit * nsolve * 2 * 2 * stride, "tensor")
+        w["k_inc_recover"] = (6 * NZ * modes * c, nsolve * NZ * 2 * 22, "fp64")
+    return w
+
+
 # which pipe bounds each kernel's counted flops: the exact GEMMs' digit
 # products run on the bf16 tensor pipe; the curl recurrences, the recovery and
 # every kernel of the FP64 path count FP64 operations; the mixed path's FP32
@@ -222,9 +265,9 @@ def step_roofline(work, precision, ms_per_step, hbm_gbs, tensor_tflops, fp64_tfl
     back).  `work` maps kernel -> (bytes, flops) per step."""
     per = {}
     total = 0.0
-    for k, (nb, nf) in work.items():
+    for k, (nb, nf, *named) in work.items():  # a third entry names the pipe
         t_mem = nb / (hbm_gbs * 1e9)
-        if k in TENSOR_KERNELS:
+        if k in TENSOR_KERNELS or named == ["tensor"]:
             t_fl, pipe = nf / (tensor_tflops * 1e12), "tensor"
         elif precision == "fp64" or k in FP64_MIXED_KERNELS:
             t_fl, pipe = nf / (fp64_tflops * 1e12), "fp64"
@@ -475,10 +518,12 @@ def main():
         return 0
     # ---- roofline of the dominant kernel
     work = kernel_work(cfg, args.zpad, args.precision, recover_df="double-float recovery" in tuning)
+    if args.precision == "fp64":
+        work.update(digit_work(cfg, args.zpad, {k for k in prof if prof[k][0] > 0}))
     kname = max((k for k in prof if prof[k][0] > 0), key=lambda k: prof[k][1])
     launches, kms = prof[kname]
     avg_ms = kms / launches
-    nbytes, nflops = work.get(kname, (0, 0))
+    nbytes, nflops, *pipe = work.get(kname, (0, 0))
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -500,8 +545,16 @@ def main():
                                      peaks.get("bf16_tflops_sustained", 1700.0), fp64_peak)
     roofline["step"]["peaks"] = ("HBM: MEASURED_PEAKS.json hbm_gbs; tensor: bf16_tflops_sustained "
                                  "(measured); FP64: cuBLAS DGEMM 4096^3 measured in this run")
-    if args.precision == "fp64":
-        # the FP64 path's kernels are bound by the FP64 pipe: their rate against
+    if pipe == ["tensor"]:
+        # exact digit products: 36 FP16 products per FP64 product
+        tensor_peak = peaks.get("bf16_tflops_sustained", 1700.0)
+        rate = nflops / (avg_ms / 1e3) / 1e12
+        roofline.update({"bound": "tensor", "achieved": rate, "peak": tensor_peak, "unit": "TFLOP/s",
+                         "frac": rate / tensor_peak, "hbm_gbs_achieved": achieved_gbs,
+                         "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained (measured); "
+                                        "the kernel's mma.sync instructions sustain 595 TFLOP/s"})
+    elif args.precision == "fp64":
+        # the FP64 path's other kernels are bound by the FP64 pipe: their rate against
         # the measured DGEMM peak
         roofline.update({"fp64_tflops_achieved": nflops / (avg_ms / 1e3) / 1e12,
                          "fp64_tflops_peak": fp64_peak,
