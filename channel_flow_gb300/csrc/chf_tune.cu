@@ -10,13 +10,11 @@
 //     rule's order, its reverse and the odd radices first, where the rule is
 //     the largest radices (16, 8, 9, ...) for the x / y lines and 4s, then
 //     2, 3, 5 for the wall-normal ones; the x / y lines also try radices up to 4;
-//   * the lines per CTA of the shared-memory FFT kernels (y: streamwise
-//     modes per CTA; x: rows per CTA; FP64 z: modes per CTA), every shape the
-//     launch rules accept;
+//   * the lines per CTA of the two-buffer FFT kernels (y: streamwise modes per
+//     CTA; x: rows per CTA; FP64 z: modes per CTA), every shape the launch
+//     rules accept, against the in-place kernels or digit products of the rule;
 //   * the increment solve's thread mapping (CHF_MIXED): modes per CTA (2 or
-//     4), matrix columns per load batch (2, 3 or 4), block rows per thread
-//     (1 or 2) and, where one row per thread at 288 threads would loop, one
-//     pass in wide blocks or the loop.
+//     4), matrix columns per load batch (2, 3 or 4) and rows per thread (1 or 2).
 // Every candidate computes the same results bit for bit (a plan change
 // rewrites the plan's stage twiddle table first, with the same values).  The
 // recovery's arithmetic (chf_set_launch_shape "recover_form") is not

@@ -28,6 +28,12 @@
 //            (REF:1502-1540), the (0,0)-mode histories (REF:1482-1487, 1560-1569)
 //            and coefficients -> Gauss-Lobatto values (REF:1573-1609).
 // The history swap of REF:1542-1558 is a pointer exchange on the host.
+//
+// These kernels are the shared-memory FFTs of every pass and the register FFTs
+// of 192-point lines.  FP64 lines of at most 384 points (512 product intervals
+// in z) run as digit products instead (k_dft64.cu), and FP32 lines of other
+// lengths than 192 in place (k_xy.cu); what is left to the FFTs here is longer
+// lines, chosen launch shapes ("kxb", "xr") and x grids of few rows.
 #include <algorithm>
 #include <cstdio>
 

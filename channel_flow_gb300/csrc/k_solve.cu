@@ -25,6 +25,13 @@
 //  * The (0,0) operator equals the omega_y operator at k^2 = 0, so the mean
 //    mode is the last "group" with k^2 = 0 and reuses the same code path; its
 //    inverse replaces the per-step full-pivot elimination of gsij.
+//
+// Who runs it: the (0,0) mode of every precision, every mode of
+// CHF_MIXED_F64SOLVE, and of CHF_FP64 where the modes are too few for
+// k_solve64.cu.  One CTA per (0,0) mode, then one per run of at most two modes
+// of a group: the FP64 pipe bounds the kernel at large grids (1254 us at 128 x
+// 129 x 128), and small ones have more CTAs than with one per group (32^3: 94
+// -> 37 us).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -788,16 +788,19 @@ int setup_inc_items(Handle* h) {
   return CHF_OK;
 }
 
-// Modes per CTA.  Two where a field has at most 160 rows: half the shared
-// memory and 56 registers a thread let 7 blocks of 160 threads run on an SM
-// (5 with four modes), and the runs of one group still share its operators
-// through L2.  Longer columns are closer to the memory rate, where the second
-// read of the operators costs more than the blocks in flight give.  Two
-// against four: 33 rows 12 / 15 us (32 x 33 x 32), 97 rows 160 / 158 us
-// (160 x 97 x 120), 129 rows 209 / 221 us (128 x 129 x 128), 193 rows 3245 /
-// 3089 us (384 x 193 x 384).
+// Modes per CTA.  Four read the operators and compute a row's exponent once
+// for more products; two, with half the shared memory and 56 registers a
+// thread, are shorter CTAs, which is better where there are few of them (under
+// 16 per SM), and let more threads run where a field fills five warps (129 to
+// 160 rows: 7 CTAs per SM against 5).  Two against four: 33 rows 12 / 15 us
+// (32 x 33 x 32), 96 channels of 33 to 97 rows one after another 133 / 136 us a
+// step, 129 rows 209 / 221 us (128 x 129 x 128); but 97 rows 160 / 158 us
+// (160 x 97 x 120), 193 rows 3245 / 3089 us (384 x 193 x 384), and the 96
+// channels stacked in six classes 56.7 / 55.4 us a channel-step.
 int inc_modes(const Handle* h) {
-  return h->tune.inc_mch ? h->tune.inc_mch : h->d.NZ <= 160 ? 2 : 4;
+  if (h->tune.inc_mch) return h->tune.inc_mch;
+  const int NZ = h->d.NZ;
+  return NZ <= 160 && (NZ > 128 || 2 * h->n_inc_items[1] < 16 * h->num_sms) ? 2 : 4;
 }
 
 int launch_recover(Handle* h, bool df) {
