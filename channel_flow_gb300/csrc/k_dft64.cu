@@ -37,9 +37,13 @@
 // Measured and not taken: tiles of 16 outputs per warp (half the reads, fewer
 // warps: 20% slower), digits kept as bytes and converted on each read (5%
 // slower), the matrix digits of the next step loaded ahead (equal), 5 or 6
-// CTAs per SM at fewer registers (equal).
+// CTAs per SM at fewer registers (equal), the last tiles' steps dealt to all four
+// warps (4% slower), the Lamb products in TF_XFWD's loads (437 -> 634 us for the
+// two), integer instead of FP64-pipe conversions of the outputs (5% slower).
+// Parts switched off in TF_XINV, of 632 us: loads 46, digits 50, stores 110
+// (conversions 40), products 280.
 // At 128 x 129 x 128 (product grid 200), against the FFT kernels: z inverse
-// 1.52 -> 0.30 ms, y inverse 0.68 -> 0.40, x with products 1.92 -> 1.06, y
+// 1.52 -> 0.30 ms, y inverse 0.68 -> 0.40, x with products 1.92 -> 1.04, y
 // forward 0.36 -> 0.25, z forward with curl and Gauss-Lobatto values 1.17 ->
 // 0.32; the errors against 64 bits of every array are equal or smaller (grids
 // of 4 to 192 points a side).
@@ -155,6 +159,25 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) k_tf(const __grid_constan
       if (m > k) v = src[(size_t)m * stride];
     }
   };
+  // u, v of k0 .. k0 + 7 of a real line (TF_XFWD), two points per load (nine
+  // loads for sixteen: 350 -> 322 us at 128 x 129 x 128).  L is even, so the
+  // mirrors of an odd k and the even one above it make an aligned pair.
+  auto fetch_pairs = [&](int k0, double (&u)[8], double (&v)[8]) {
+    const int last = live ? sh.k_e - 1 : -1, m0 = sh.L - k0;  // last = L / 2, its own mirror
+    const double2* pairs = reinterpret_cast<const double2*>(src);
+    double2 a[4], b[5];  // points k0 + 2 i, + 1; points m0 - 2 i, + 1
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = k0 + 2 * i <= last ? pairs[(k0 >> 1) + i] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+      b[i] = k0 + 2 * i > 0 && k0 + 2 * i - 1 <= last ? pairs[(m0 >> 1) - i] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int k = k0 + i;
+      u[i] = k <= last ? ((i & 1) ? a[i >> 1].y : a[i >> 1].x) : 0.0;
+      v[i] = k > 0 && k < last ? ((i & 1) ? b[(i + 1) >> 1].y : b[i >> 1].x) : 0.0;
+    }
+  };
   // 16-byte piece of (plane, octet of k) of the thread's line; O octets follow E's
   auto piece = [&](int plane, int octet) {
     return (plane * KS + (octet >> 1)) * 32 + (octet & 1) * 16 + slot;
@@ -168,8 +191,12 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) k_tf(const __grid_constan
   int emax = 0;
   for (int o = tid >> 4; o < octs; o += TF_THREADS / 16) {
     double u[8], v[8];
+    if constexpr (MODE == TF_XFWD) {
+      fetch_pairs(8 * o, u, v);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) fetch(8 * o + i, u[i], v[i]);
+      for (int i = 0; i < 8; ++i) fetch(8 * o + i, u[i], v[i]);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       emax = max(emax, max((__double2hiint(u[i]) >> 20) & 0x7ff, (__double2hiint(v[i]) >> 20) & 0x7ff));
