@@ -13,8 +13,8 @@
 // with w_kx = 1 for kx = 0 and 2 for kx > 0 (the half spectrum in x), and
 // <f>(z_k) = Re f^_{00}(z_k).  The only transform is Chebyshev coefficients
 // -> Gauss-Lobatto values, as exact digit products (k_dft64.cu).  A whole call
-// at 128^3 takes 202 us, with the FFTs of these lines it took 466; at 32^3
-// 47 / 58 us.
+// at 128^3 takes 182 us, with the FFTs of these lines and weights in the sums it
+// took 466; at 32^3 48 / 58 us.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -38,40 +38,54 @@ __global__ void __launch_bounds__(ST_THREADS) k_stat_sum(const cd* __restrict__ 
   const cd* U = gl + ((size_t)0 * NZ + k) * modes;
   const cd* V = gl + ((size_t)1 * NZ + k) * modes;
   const cd* W = gl + ((size_t)2 * NZ + k) * modes;
-  double acc[7] = {0, 0, 0, 0, 0, 0, 0};  // uu vv ww uv uw vw energy
-  for (long m = threadIdx.x; m < modes; m += blockDim.x) {
-    const int kx = (int)(m % d.KX), ky = (int)(m / d.KX);
-    if (ky == d.NYQ) continue;
-    const double wt = kx == 0 ? 1.0 : 2.0;
+  // uu vv ww uv uw vw, the modes of kx = 0 (weight 1) before those of kx > 0
+  // (weight 2): 12 FP64 operations per mode and no weight to multiply
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  auto add = [&](long m) {
     const cd a = U[m], b = V[m], c = W[m];
-    const double ea = a.re * a.re + a.im * a.im, eb = b.re * b.re + b.im * b.im, ec = c.re * c.re + c.im * c.im;
-    acc[6] += wt * (ea + eb + ec);
-    if (m == 0) continue;  // the mean mode is not a fluctuation
-    acc[0] += wt * ea;
-    acc[1] += wt * eb;
-    acc[2] += wt * ec;
-    acc[3] += wt * (a.re * b.re + a.im * b.im);
-    acc[4] += wt * (a.re * c.re + a.im * c.im);
-    acc[5] += wt * (b.re * c.re + b.im * c.im);
+    acc[0] = fma(a.re, a.re, fma(a.im, a.im, acc[0]));
+    acc[1] = fma(b.re, b.re, fma(b.im, b.im, acc[1]));
+    acc[2] = fma(c.re, c.re, fma(c.im, c.im, acc[2]));
+    acc[3] = fma(a.re, b.re, fma(a.im, b.im, acc[3]));
+    acc[4] = fma(a.re, c.re, fma(a.im, c.im, acc[4]));
+    acc[5] = fma(b.re, c.re, fma(b.im, c.im, acc[5]));
+  };
+  const long nyq0 = (long)d.NYQ * d.KX, nyq1 = nyq0 + d.KX;  // the spanwise Nyquist slot is left out
+  double zero[6];
+  for (int ky = threadIdx.x; ky < d.KY; ky += blockDim.x)
+    if (ky != d.NYQ && ky > 0) add((long)ky * d.KX);  // (0, 0) is not a fluctuation
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    zero[q] = acc[q];
+    acc[q] = 0.0;
   }
-  __shared__ double red[ST_THREADS / 32][7];
+  for (long m = threadIdx.x; m < modes; m += blockDim.x)
+    if ((unsigned int)m % (unsigned int)d.KX != 0 && (m < nyq0 || m >= nyq1)) add(m);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) acc[q] = fma(2.0, acc[q], zero[q]);
+  __shared__ double red[ST_THREADS / 32][6];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < 7; ++q) {
+  for (int q = 0; q < 6; ++q) {
     double x = acc[q];
     for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
     if (lane == 0) red[warp][q] = x;
   }
   __syncthreads();
-  if (threadIdx.x < 7) {
+  if (threadIdx.x < 6) {
     double x = 0.0;
     for (int q = 0; q < ST_THREADS / 32; ++q) x += red[q][threadIdx.x];
     out[(size_t)k * NSTAT + 3 + threadIdx.x] = x;
+    red[0][threadIdx.x] = x;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    out[(size_t)k * NSTAT + 0] = U[0].re;
-    out[(size_t)k * NSTAT + 1] = V[0].re;
-    out[(size_t)k * NSTAT + 2] = W[0].re;
+    const cd a = U[0], b = V[0], c = W[0];
+    out[(size_t)k * NSTAT + 0] = a.re;
+    out[(size_t)k * NSTAT + 1] = b.re;
+    out[(size_t)k * NSTAT + 2] = c.re;
+    const double mean = (a.re * a.re + a.im * a.im) + (b.re * b.re + b.im * b.im) + (c.re * c.re + c.im * c.im);
+    out[(size_t)k * NSTAT + 9] = mean + red[0][0] + red[0][1] + red[0][2];
   }
 }
 
