@@ -208,9 +208,11 @@ int chf_tuning(const chf_handle* h, char* buf, int len);
  *                  float where the grid has at least 16 x 32 x SMs / 4
  *                  modes).  The one setting whose results differ (in the
  *                  last bits); the autotuner leaves it alone.
- *   "kxb", "xr", "zl_c2v", "zl_curl"  lines per CTA of the shared-memory
- *                  FFT kernels: one of the shapes that fit the grid, or 0
- *                  for the launcher's rule
+ *   "kxb", "xr", "zl_c2v", "zl_curl"  lines per CTA of the two-buffer FFT
+ *                  kernels: one of the shapes that fit the grid, or 0 for
+ *                  the launcher's rule (CHF_MIXED x / y lines: in place).
+ *                  Without effect where CHF_FP64 transforms by digit
+ *                  products (x / y lines up to 384 points, z up to 512)
  * CHF_E_INVALID for an unknown name or a value that the grid or the other
  * shapes rule out (the handle is then unchanged).  Synchronous. */
 int chf_set_launch_shape(chf_handle* h, const char* name, int value);
