@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) k_tf(const __grid_constan
   double* out = a.out[f];
   const uint4 *mat_e = a.mat + lane, *mat_o = mat_e + (size_t)sh.tiles_e * sh.ks_e * 128;
   for (int tile = warp; tile < sh.tiles_e; tile += TF_THREADS / 32) {  // tiles_o <= tiles_e
+    __syncwarp();  // lanes without a line left the last tile's stores early; ldmatrix and mma take whole warps
     long long E[4], O[4];
     sums(0, sh.ks_e, mat_e + (size_t)tile * sh.ks_e * 128, E);
     sums(sh.ks_e, tile < sh.tiles_o ? sh.ks_o : 0, mat_o + (size_t)tile * sh.ks_o * 128, O);

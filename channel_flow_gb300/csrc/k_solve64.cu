@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
   const long mode = s_mode[q];
   const short4* gexp = reinterpret_cast<const short4*>(a.exps) + (size_t)grp * sh.strips * 8 + row;
   for (int s = warp; s < sh.strips; s += S64_THREADS / 32) {
+    __syncwarp();  // lanes without a mode left the last strip's stores early; mma takes whole warps
     int blk = 0;
     while (blk < 3 && s >= sh.strip0[blk + 1]) ++blk;
     const int i = s - sh.strip0[blk], par = blk & 1, T = sh.tiles[par], n = sh.n[par];

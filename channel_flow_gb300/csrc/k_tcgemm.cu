@@ -412,6 +412,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_gemm_fx(const __grid_const
                           (reinterpret_cast<uintptr_t>(out) & (2 * sizeof(OutT) - 1)) == 0;
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {  // rows 16 hf .. 16 hf + 15 of the quarter
+        __syncwarp();  // lanes past the last row left the stores early; tcgen05.ld takes whole warps
         uint32_t r[NP][16];
 #pragma unroll
         for (int L = 0; L < NP; ++L) {
