@@ -308,25 +308,34 @@ int transform_dev(Handle* h, int isign, cd* buf) {
 }
 
 // First use: three field-sized buffers and NZ x 3 plane maxima, the nnx- and
-// nny-point plans and their twiddles.
+// nny-point plans and their twiddles.  phys_buf says that all of them are
+// there: it is set last, and a failed set-up leaves nothing behind.
 int ensure_phys(Handle* h) {
   if (h->phys_buf) return CHF_OK;
   const Dims& d = h->d;
   const size_t fb = sizeof(cd) * d.field_elems();
-  if (!cuda_ok(h, cudaMalloc(&h->phys_buf, 3 * fb + sizeof(double) * 3 * (size_t)d.NZ), "physical buffers"))
-    return CHF_E_NOMEM;
   h->pxu = make_plan(d.nnx);
   h->pyu = make_plan(d.nny);
-  struct {
-    cd** dst;
-    int L;
-  } tws[] = {{&h->tw_pxu, d.nnx}, {&h->tw_pyu, d.nny}};
-  for (auto& t : tws) {
-    std::vector<cd> v = twiddles(t.L);
-    if (!cuda_ok(h, cudaMalloc((void**)t.dst, sizeof(cd) * v.size()), "twiddle alloc") ||
-        !cuda_ok(h, cudaMemcpy(*t.dst, v.data(), sizeof(cd) * v.size(), cudaMemcpyHostToDevice), "twiddle upload"))
-      return CHF_E_CUDA;
+  void* buf = nullptr;
+  cd* tw[2] = {nullptr, nullptr};
+  const int L[2] = {d.nnx, d.nny};
+  int rc = cuda_ok(h, cudaMalloc(&buf, 3 * fb + sizeof(double) * 3 * (size_t)d.NZ), "physical buffers") ? CHF_OK
+                                                                                                       : CHF_E_NOMEM;
+  for (int i = 0; i < 2 && rc == CHF_OK; ++i) {
+    std::vector<cd> v = twiddles(L[i]);
+    if (!cuda_ok(h, cudaMalloc((void**)&tw[i], sizeof(cd) * v.size()), "twiddle alloc") ||
+        !cuda_ok(h, cudaMemcpy(tw[i], v.data(), sizeof(cd) * v.size(), cudaMemcpyHostToDevice), "twiddle upload"))
+      rc = CHF_E_CUDA;
   }
+  if (rc != CHF_OK) {
+    cudaFree(buf);
+    for (cd* t : tw) cudaFree(t);
+    cudaGetLastError();  // or the next launch's check would report it again
+    return rc;
+  }
+  h->tw_pxu = tw[0];
+  h->tw_pyu = tw[1];
+  h->phys_buf = buf;
   return CHF_OK;
 }
 

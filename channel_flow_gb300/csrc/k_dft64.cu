@@ -606,7 +606,10 @@ struct TfItem {
   int mode, period;
 };
 
-// the digit matrices of the items' plans, in one allocation *image
+// the digit matrices of the items' plans, in one allocation.  *image says that
+// they are there (setup_tf, setup_tf_out), so it and the plans' pointers are set
+// after the last step of the set-up has succeeded; a failed one leaves them null
+// and is done again by the next call.
 int build_tf(Handle* h, const std::vector<TfItem>& items, void** image) {
   size_t vecs = 0, entries = 0;
   for (const TfItem& it : items) {
@@ -622,28 +625,42 @@ int build_tf(Handle* h, const std::vector<TfItem>& items, void** image) {
     host.insert(host.end(), cs.begin(), cs.end());
     host.insert(host.end(), sn.begin(), sn.end());
   }
-  if (!cuda_ok(h, cudaMalloc(image, sizeof(uint4) * vecs + sizeof(long long) * entries), "transform digits"))
+  void* mem = nullptr;
+  if (!cuda_ok(h, cudaMalloc(&mem, sizeof(uint4) * vecs + sizeof(long long) * entries), "transform digits")) {
+    cudaGetLastError();
     return CHF_E_NOMEM;
-  uint4* mat = static_cast<uint4*>(*image);
-  const long long* tab = reinterpret_cast<const long long*>(mat + vecs);
-  if (!cuda_ok(h, cudaMemcpyAsync((void*)tab, host.data(), sizeof(long long) * entries, cudaMemcpyHostToDevice, h->stream),
-               "transform tables"))
-    return CHF_E_CUDA;
+  }
+  uint4* const first = static_cast<uint4*>(mem);
+  const long long* tab = reinterpret_cast<const long long*>(first + vecs);
+  bool good = cuda_ok(h, cudaMemcpyAsync((void*)tab, host.data(), sizeof(long long) * entries, cudaMemcpyHostToDevice,
+                                         h->stream),
+                      "transform tables");
+  uint4* mat = first;
   for (const TfItem& it : items) {
+    if (!good) break;
     const TfShape& s = it.p->s;
-    it.p->mat = mat;
     const int blocks = (int)((tf_mat_vecs(s) / 128 + 3) / 4);
     const long long *cs = tab, *sn = tab + it.period;
     if (it.mode == TF_Z) k_tf_matrix<TF_Z><<<blocks, 128, 0, h->stream>>>(cs, sn, s, it.period, mat);
     else if (it.mode == TF_Z2) k_tf_matrix<TF_Z2><<<blocks, 128, 0, h->stream>>>(cs, sn, s, it.period, mat);
     else if (it.mode == TF_XINV) k_tf_matrix<TF_XINV><<<blocks, 128, 0, h->stream>>>(cs, sn, s, it.period, mat);
     else k_tf_matrix<TF_YINV><<<blocks, 128, 0, h->stream>>>(cs, sn, s, it.period, mat);
+    good = cuda_ok(h, cudaGetLastError(), "k_tf_matrix");
     mat += tf_mat_vecs(s);
     tab += 2 * it.period;
   }
-  if (!cuda_ok(h, cudaGetLastError(), "k_tf_matrix") ||
-      !cuda_ok(h, cudaStreamSynchronize(h->stream), "transform tables"))
+  good = good && cuda_ok(h, cudaStreamSynchronize(h->stream), "transform tables");
+  if (!good) {
+    cudaFree(mem);
+    cudaGetLastError();  // or the next launch's check would report it again
     return CHF_E_CUDA;
+  }
+  mat = first;
+  for (const TfItem& it : items) {
+    it.p->mat = mat;
+    mat += tf_mat_vecs(it.p->s);
+  }
+  *image = mem;
   return CHF_OK;
 }
 
