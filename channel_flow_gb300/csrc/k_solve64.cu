@@ -18,6 +18,12 @@
 // the AB2 term of up to four modes of one k^2 (eight real columns, an n8
 // operand) and multiplies.  The digits lose 2^-62 of the row's and of the
 // column's largest value and the dropped levels about 2^-58 of their product.
+// That is a loss only where the largest entry of a row takes no part: the
+// columns of A^-1 that belong to the wall rows meet zeros (r vanishes there) but
+// exceed v's other columns by 2^8 to 2^16 at large k^2, so they are left out of
+// the digits.  With them A^-1 r came out 1e-14 to 1e-12 off (k^2 = 1e2 to 3e4,
+// 128 intervals, dt 2e-4, re 180; relative to its largest value), without them
+// 1e-17; plain FP64 gives 1e-16 (M c: 1e-17 against 1e-16).
 //
 // A CTA takes one run of at most 4 modes of one k^2 group (setup_inc_items).
 // Warp (field, mode) reads the mode's coefficients and histories of one field
@@ -361,13 +367,14 @@ __global__ void __launch_bounds__(256) k_digits_solve64(const double* __restrict
   const BlockOffsets bo = block_offsets(sl);
   const size_t off = blk == 0 ? bo.ve : blk == 1 ? bo.vo : blk == 2 ? bo.we : bo.wo;
   const double* src[2] = {minc + (size_t)gl * sl.stride + off, xinv + (size_t)g * sl.stride + off};
+  const int first[2] = {0, blk < 2 ? 2 : 1};  // A^-1's columns of the wall rows, whose r is zero, stay out
   if (tid < 32) s_e[tid >> 4][tid & 15] = 0;
   __syncthreads();
   for (int op = 0; op < 2; ++op) {
     const int r = 16 * i + (tid & 15);
     int e = 0;
     if (r < cols)
-      for (int c = tid >> 4; c < cols; c += 16) e = max(e, biased_exp(src[op][(size_t)c * n + r]));
+      for (int c = first[op] + (tid >> 4); c < cols; c += 16) e = max(e, biased_exp(src[op][(size_t)c * n + r]));
     atomicMax(&s_e[op][tid & 15], e);
   }
   __syncthreads();
@@ -384,7 +391,7 @@ __global__ void __launch_bounds__(256) k_digits_solve64(const double* __restrict
       long long x[4];
       for (int c = 0; c < 4; ++c) {
         const int k = 16 * kt + 2 * (lane & 3) + (c & 1) + 8 * (c >> 1);
-        const double v = r < cols && k < cols ? src[op][(size_t)k * n + r] : 0.0;
+        const double v = r < cols && k >= first[op] && k < cols ? src[op][(size_t)k * n + r] : 0.0;
         x[c] = fixed_of((uint32_t)__double2loint(v), (uint32_t)__double2hiint(v), s_e[op][lane / 4 + 8 * h]);
       }
       digit_bytes(x, w[h]);
