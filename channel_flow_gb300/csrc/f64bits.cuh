@@ -128,11 +128,15 @@ __host__ __device__ __forceinline__ double widen(float f) {
   return u2d(sign | (ed << 52) | ((uint64_t)(v & 0x7fffffu) << 29));
 }
 
-// x / 2 by decrementing the exponent (exact for |x| >= 2^-1021; smaller
-// magnitudes give signed zero)
+// x / 2 on the bits, as x * 0.5 gives it: the exponent less one; infinity and
+// NaN stay what they are (less one they would be finite), and below 2^-1021 the
+// significand is halved instead, ties to even
 __host__ __device__ __forceinline__ double half(double x) {
-  const uint64_t u = d2u(x);
-  return ((u >> 52) & 0x7ff) > 1 ? u2d(u - (1ull << 52)) : u2d(u & 0x8000000000000000ull);
+  const uint64_t u = d2u(x), m = u & 0x7fffffffffffffffull;
+  const int e = (int)(m >> 52);
+  if (e == 0x7ff) return x;
+  if (e > 1) return u2d(u - (1ull << 52));
+  return u2d((u & 0x8000000000000000ull) | ((m >> 1) + ((m >> 1) & m & 1)));
 }
 
 // the binary64 of an integer 1 <= n < 2^31 (exact)
