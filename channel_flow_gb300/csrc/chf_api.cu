@@ -15,6 +15,19 @@ bool cuda_ok(Handle* h, cudaError_t e, const char* what) {
   return false;
 }
 
+// Whether the device has `bytes` for something that the handle can do without,
+// and then still the buffers that later calls allocate: at most the state
+// saved by chf_autotune, five fields of the pressure and three each of the
+// statistics and the physical velocity.
+bool spare_memory(const Handle* h, size_t bytes) {
+  size_t avail = 0, total = 0;
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return avail >= bytes + 20 * sizeof(cd) * h->d.field_elems() + (size_t(64) << 20);
+}
+
 FftPlan make_plan(int L) {
   FftPlan p{};
   p.L = L;
@@ -186,7 +199,7 @@ static void release(chf_handle* h) {
   if (h->device >= 0) cudaSetDevice(h->device);
   for (auto& p : h->f) cudaFree(p);
   for (auto& p : h->mean) cudaFree(p);
-  void* ptrs[] = {h->iapha, h->ibeta, h->t0, h->t2, h->t4, h->k2vals, h->xinv, h->xmean,
+  void* ptrs[] = {h->iapha, h->ibeta, h->t0, h->t2, h->t4, h->k2vals, h->xinv,
                   h->group_start, h->group_modes, h->tw_py, h->tw_px, h->tw_z2, h->tw_zm,
                   h->twf_py, h->twf_px, h->stw_py, h->stw_px, h->stw_py64, h->stw_px64, h->place_py, h->place_px, h->incm, h->incx, h->incr_exp, h->inc_items, h->s64_mat, h->s64_exp, h->s64_ext, h->phi, h->flow, h->stats_buf, h->pres_buf, h->phys_buf, h->tw_pxu, h->tw_pyu, h->group_re, h->ubphi_dev, h->wz, h->wy, h->wp, h->tf_image, h->tf_out_image, h->scratch, h->dev_status, h->az1, h->az2,
                   h->agl, h->bimg, h->wz32, h->wy32, h->lc64, h->aexp1, h->aexp2, h->aexp3, h->bexp, h->z2_tail, h->gl_tail};
@@ -340,10 +353,8 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
     const size_t wz_elems = (size_t)6 * d.MP * d.modes();
     const size_t wy_elems = (size_t)6 * d.MP * d.PY * d.KX;
     if (!cuda_ok(h, cudaMalloc((void**)&h->wz, sizeof(cd) * wz_elems), "work alloc") ||
-        !cuda_ok(h, cudaMalloc((void**)&h->wy, sizeof(cd) * wy_elems), "work alloc") ||
-        (tf_xy(d) && !cuda_ok(h, cudaMalloc((void**)&h->wp, sizeof(double) * tf_phys_elems(d)), "work alloc")))
+        !cuda_ok(h, cudaMalloc((void**)&h->wy, sizeof(cd) * wy_elems), "work alloc"))
       return fail(CHF_E_NOMEM);
-    if (const int rc = setup_tf(h); rc != CHF_OK) return fail(rc);
   }
   if (!cuda_ok(h, cudaMalloc((void**)&h->dev_status, sizeof(int)), "status alloc") ||
       !cuda_ok(h, cudaMemsetAsync(h->dev_status, 0, sizeof(int), h->stream), "status init"))
@@ -374,7 +385,7 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
   if (rc != CHF_OK) return fail(rc);
   if (mixed_front(h)) rc = setup_mixed(h);
   if (rc == CHF_OK) rc = setup_inc_items(h);
-  if (rc == CHF_OK) rc = increment_solve(h) ? setup_solver_mixed(h) : setup_solve64(h);
+  if (rc == CHF_OK && increment_solve(h)) rc = setup_solver_mixed(h);
   if (rc != CHF_OK) return fail(rc);
   if (!cuda_ok(h, cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking), "cudaStreamCreate") ||
       !cuda_ok(h, cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming), "cudaEventCreate") ||
@@ -387,12 +398,19 @@ int chf_create(const chf_config* cfg, chf_handle** out) {
     if (!cuda_ok(h, cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate")) return fail(CHF_E_CUDA);
   for (cudaEvent_t& e : h->ev_field)
     if (!cuda_ok(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate")) return fail(CHF_E_CUDA);
+  // what CHF_FP64 can do without comes last: its solve's operators as digits,
+  // then the transforms' (with three physical fields of work space)
+  if (cfg->precision == CHF_FP64) {
+    rc = setup_solve64(h);
+    if (rc == CHF_OK) rc = setup_tf(h);
+    if (rc != CHF_OK) return fail(rc);
+  }
   // FP64: k_zc2v, k_yinv, k_xprod, k_yfwd, k_zcurl (as digit
   // products: x in three kernels, and k_zcurl as k_tf, k_curl64, k_tf and
   // k_meanfix); mixed front:
   // two splits, three GEMMs, k_yinv_w, k_xprod_w, k_yfwd_w, k_curl,
   // k_meanfix; then k_solve, or the modes' solve, k_inc_recover and the (0,0) mode
-  h->kernels_per_step = (mixed_front(h) ? 10 : 5 + (tf_xy(d) ? 2 : 0) + (tf_z(d) ? 3 : 0)) +
+  h->kernels_per_step = (mixed_front(h) ? 10 : 5 + (tf_xy(h) ? 2 : 0) + (tf_z(h) ? 3 : 0)) +
                         (increment_solve(h) || solve64(h) ? 3 : 1);
   if (!cuda_ok(h, cudaStreamSynchronize(h->stream), "create sync")) return fail(CHF_E_CUDA);
   *out = h;

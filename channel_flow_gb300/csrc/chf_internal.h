@@ -158,7 +158,8 @@ struct Handle {
   SolveLayout sl{};
   int nk2 = 0;
   double* k2vals = nullptr;   // nk2
-  double* xinv = nullptr;     // nk2 * sl.stride
+  double* xinv = nullptr;     // inverses of groups xinv_first .. nk2 (the (0,0) mode), sl.stride each
+  int xinv_first = 0;         // nk2 where only the (0,0) mode's is kept (setup_solve64)
   // mixed solve (k_solve_mixed.cu), per k^2: A^-1 (B - A) as (hi, lo)
   // floats, A^-1 as floats, and per row the exponent of sum |hi| over the row
   float2* incm = nullptr;
@@ -175,7 +176,6 @@ struct Handle {
   short* s64_exp = nullptr;
   double* s64_ext = nullptr;
   bool rec_df_rule = false;  // k_inc_recover's double-float form (setup_solver_mixed)
-  double* xmean = nullptr;    // inverse of the (0,0) operator, NZ x NZ column-major
   int* group_start = nullptr; // nk2 + 1 (modes grouped by k^2)
   int* group_modes = nullptr; // solved modes, sorted by k^2 index
   int nsolve = 0;
@@ -305,6 +305,7 @@ void prof_begin(Handle* h, int kid, cudaEvent_t* a);
 void prof_end(Handle* h, int kid, cudaEvent_t a);
 
 bool cuda_ok(Handle* h, cudaError_t e, const char* what);
+bool spare_memory(const Handle* h, size_t bytes);
 
 // launchers (k_nonlinear.cu)
 int launch_nonlinear_fp64(Handle* h);
@@ -361,9 +362,8 @@ bool xy_register_path(const Dims& d);
 int launch_yinv_fields(Handle* h, cf* wz, cf* wy, const cf* tw_py, int f0, int nf);
 int launch_xprod_yfwd(Handle* h, cf* wz, cf* wy, const cf* tw_py, const cf* tw_px);
 // FP64 transforms as exact digit products (k_dft64.cu)
-bool tf_z(const Dims& d);
-bool tf_xy(const Dims& d);
-size_t tf_phys_elems(const Dims& d);  // of wp
+bool tf_z(const Handle* h);   // after setup_tf: they serve the wall-normal,
+bool tf_xy(const Handle* h);  // the in-plane transforms
 int setup_tf(Handle* h);
 int launch_tf_c2v(Handle* h);
 int launch_tf_xy(Handle* h);
@@ -380,7 +380,7 @@ int launch_y_in_place(Handle* h, cf* wz, cf* wy, const FftPlan& py, const cf* st
                       bool inverse);
 int launch_x_in_place(Handle* h, cf* wy, const FftPlan& px, const cf* stab, const unsigned short* tab);
 int launch_solve_fp64(Handle* h);  // k_solve.cu
-bool solve64(const Handle* h);     // k_solve64.cu
+bool solve64(const Handle* h);     // k_solve64.cu, after setup_solve64
 int setup_solve64(Handle* h);
 int launch_solve64(Handle* h);
 int launch_recover(Handle* h, bool df);  // k_solve_mixed.cu: u, w, omega_x, omega_z from v, omega_y

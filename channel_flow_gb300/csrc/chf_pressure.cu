@@ -279,13 +279,11 @@ extern "C" int chf_pressure(chf_handle* h, double* p_out) {
   if (!h->wy &&
       !cuda_ok(h, cudaMalloc((void**)&h->wy, sizeof(cd) * 6 * (size_t)d.MP * d.PY * d.KX), "pressure work"))
     return CHF_E_NOMEM;
-  if (!h->wp && tf_xy(d) &&
-      !cuda_ok(h, cudaMalloc((void**)&h->wp, sizeof(double) * tf_phys_elems(d)), "pressure work"))
-    return CHF_E_NOMEM;
-  if (const int rc = setup_tf(h); rc != CHF_OK) return rc;
   if (!h->pres_buf &&
       !cuda_ok(h, cudaMalloc(&h->pres_buf, sizeof(cd) * 5 * (size_t)NZ * modes + sizeof(int)), "pressure buffer"))
     return CHF_E_NOMEM;
+  if (mixed_front(h))  // last, as it can do without
+    if (const int rc = setup_tf(h); rc != CHF_OK) return rc;
   cd* hc = static_cast<cd*>(h->pres_buf);  // 3 x [NZ][modes]
   cd* R = hc + (size_t)3 * NZ * modes;
   cd* P = R + (size_t)NZ * modes;

@@ -592,9 +592,12 @@ __global__ void __launch_bounds__(CURL64_THREADS) k_curl64(const double* __restr
 // intervals 0.26 / 1.26, 0.29 / 0.71 and 0.48 / 1.14 ms (the longest that fit
 // shared memory by far); x and y on lines of 240, 300, 384 and 480 points
 // 1.07 / 1.74, 1.80 / 2.41, 2.99 / 3.33 and 5.16 / 3.91 ms.
+// A device without room for their work space (spare_memory) keeps the FFTs.
 constexpr int kTfMaxZ = 512, kTfMaxXY = 384;
-bool tf_z(const Dims& d) { return d.nch == 1 && d.MZ <= kTfMaxZ; }
-bool tf_xy(const Dims& d) { return d.nch == 1 && d.PX <= kTfMaxXY && d.PY <= kTfMaxXY; }
+static bool z_lines(const Dims& d) { return d.nch == 1 && d.MZ <= kTfMaxZ; }
+static bool xy_lines(const Dims& d) { return d.nch == 1 && d.PX <= kTfMaxXY && d.PY <= kTfMaxXY; }
+bool tf_z(const Handle* h) { return h->tf_image && z_lines(h->d); }
+bool tf_xy(const Handle* h) { return h->wp != nullptr; }
 
 // the unpadded lines of the physical velocity: the same lengths (chf_phys.cu has the figures)
 bool tf_phys(const Dims& d) { return d.nch == 1 && d.nnx <= kTfMaxXY && d.nny <= kTfMaxXY; }
@@ -666,9 +669,19 @@ int build_tf(Handle* h, const std::vector<TfItem>& items, void** image) {
 
 }  // namespace
 
+// CHF_E_NOMEM from build_tf leaves the FFTs in charge too
 int setup_tf(Handle* h) {
   const Dims& d = h->d;
-  if (!(tf_z(d) || tf_xy(d)) || h->tf_image) return CHF_OK;
+  if (h->tf_image) return CHF_OK;
+  const bool z = z_lines(d);
+  bool xy = xy_lines(d);
+  void* wp = nullptr;
+  if (xy) {
+    const size_t bytes = sizeof(double) * 6 * (size_t)d.MP * d.PY * d.PX;
+    xy = spare_memory(h, bytes) && cudaMalloc(&wp, bytes) == cudaSuccess;
+    if (!xy) cudaGetLastError();
+  }
+  if (!z && !xy) return CHF_OK;
   const int M = d.MZ, N = d.N;
   h->tf_z1.s = tf_shape(M, N / 2 + 1, N / 2, M / 2 + 1, (M + 1) / 2);
   h->tf_gl.s = tf_shape(N, N / 2 + 1, N / 2, N / 2 + 1, N / 2);
@@ -684,7 +697,14 @@ int setup_tf(Handle* h) {
                         {&h->tf_yf, TF_YFWD, d.PY},
                         {&h->tf_xi, TF_XINV, d.PX},
                         {&h->tf_xf, TF_XFWD, d.PX}};
-  return build_tf(h, std::vector<TfItem>(all + (tf_z(d) ? 0 : 3), all + (tf_xy(d) ? 7 : 3)), &h->tf_image);
+  const int rc = build_tf(h, std::vector<TfItem>(all + (z ? 0 : 3), all + (xy ? 7 : 3)), &h->tf_image);
+  if (rc == CHF_OK)
+    h->wp = static_cast<double*>(wp);
+  else
+    cudaFree(wp);
+  if (rc != CHF_E_NOMEM) return rc;
+  h->err.clear();
+  return CHF_OK;
 }
 
 // The unpadded transforms of the statistics and the physical velocity: values
@@ -726,8 +746,6 @@ int launch_tf_plane(Handle* h, cd* const* f, int n) {
   const int rc = launch_tf<TF_YINV>(h, d, h->tf_oy, x, x, n, (long)d.NZ * d.KX, -1);
   return rc != CHF_OK ? rc : launch_tf<TF_XINV>(h, d, h->tf_ox, x, x, n, (long)d.NZ * d.nny, -1);
 }
-
-size_t tf_phys_elems(const Dims& d) { return tf_xy(d) ? (size_t)6 * d.MP * d.PY * d.PX : 0; }
 
 // the six fields' values on the product grid: state -> wz
 int launch_tf_c2v(Handle* h) {

@@ -871,7 +871,7 @@ template int launch_xy<float>(Handle*, cf*, cf*, const cf*, const cf*);
 static int launch_products_fp64(Handle* h) {
   const Dims& d = h->d;
   int rc;
-  if (tf_z(d)) {
+  if (tf_z(h)) {
     rc = launch_tf_c2v(h);
   } else {
     const int zl = h->tune.zl_c2v ? h->tune.zl_c2v : pick_zl_c2v(d);
@@ -882,19 +882,19 @@ static int launch_products_fp64(Handle* h) {
     rc = zl == 8 ? run_zc2v<8>(h) : zl == 4 ? run_zc2v<4>(h) : run_zc2v<2>(h);
   }
   if (rc != CHF_OK) return rc;
-  return tf_xy(d) ? launch_tf_xy(h) : launch_xy<double>(h, h->wz, h->wy, h->tw_py, h->tw_px);
+  return tf_xy(h) ? launch_tf_xy(h) : launch_xy<double>(h, h->wz, h->wy, h->tw_py, h->tw_px);
 }
 
 int launch_nonlinear_fp64(Handle* h) {
   const Dims& d = h->d;
   const int zc = h->tune.zl_curl ? h->tune.zl_curl : pick_zl_curl(d);
-  if (!tf_z(d) && !zc) {
+  if (!tf_z(h) && !zc) {
     h->err = "z transforms: FFT length too large for the launch shapes";
     return CHF_E_INVALID;
   }
   int rc = launch_products_fp64(h);
   if (rc != CHF_OK) return rc;
-  rc = tf_z(d) ? launch_tf_curl(h) : zc == 8 ? run_zcurl<8>(h) : zc == 4 ? run_zcurl<4>(h) : run_zcurl<2>(h);
+  rc = tf_z(h) ? launch_tf_curl(h) : zc == 8 ? run_zcurl<8>(h) : zc == 4 ? run_zcurl<4>(h) : run_zcurl<2>(h);
   if (rc != CHF_OK) return rc;
   std::swap(h->f[F_U], h->f[F_RV]);
   std::swap(h->f[F_W], h->f[F_RG]);
@@ -908,7 +908,7 @@ int launch_lamb_fp64(Handle* h, cd* hc) {
   const Dims& d = h->d;
   int rc = launch_products_fp64(h);
   if (rc != CHF_OK) return rc;
-  if (tf_z(d)) {
+  if (tf_z(h)) {
     cd* c[3] = {hc, hc + (size_t)d.NZ * d.modes(), hc + (size_t)2 * d.NZ * d.modes()};
     return launch_tf_v2c(h, c);
   }

@@ -453,34 +453,63 @@ Sol64Shape solve64_shape(int N) {
 // SMs 16 x 65 x 16 131 / 125, 16 x 65 x 4 121 / 115, 24 x 21 x 12 78 / 80.
 // CHF_MIXED_F64SOLVE stays with k_solve: its FP32 front turns any change of
 // the state's last bit into another rounding of the next step.
-bool solve64(const Handle* h) {
-  return h->cfg.precision == CHF_FP64 && h->n_inc_items[0] + 1 > h->num_sms;
-}
+//
+// The digits of M and X take twice the bytes of the inverses (128 x 129 x 128:
+// 0.85 against 0.42 GB), which go once they are cut, all but the (0,0) mode's.
+// Where the device cannot hold them (spare_memory), k_solve serves as well.
+bool solve64(const Handle* h) { return h->s64_mat != nullptr; }
 
 int setup_solve64(Handle* h) {
-  if (!solve64(h)) return CHF_OK;
-  h->s64 = solve64_shape(h->d.N);
-  const size_t all = (size_t)h->nk2;
-  if (!cuda_ok(h, cudaMalloc((void**)&h->s64_mat, sizeof(uint4) * h->s64.mat_stride * all), "solve digits") ||
-      !cuda_ok(h, cudaMalloc((void**)&h->s64_exp, sizeof(short) * 32 * h->s64.strips * all), "solve digits") ||
-      !cuda_ok(h, cudaMalloc((void**)&h->s64_ext, sizeof(double) * h->s64.ext_stride * all), "solve digits"))
-    return CHF_E_NOMEM;
-  const Sol64Shape& s = h->s64;
+  if (h->cfg.precision != CHF_FP64 || h->n_inc_items[0] + 1 <= h->num_sms) return CHF_OK;
+  const Sol64Shape s = solve64_shape(h->d.N);
+  const size_t all = (size_t)h->nk2, group = sizeof(double) * h->sl.stride;
   const int chunk = std::min(h->nk2, 1024);  // groups whose M is held in FP64 at a time
-  double* minc = nullptr;
-  if (!cuda_ok(h, cudaMalloc((void**)&minc, sizeof(double) * h->sl.stride * chunk), "solve set-up")) return CHF_E_NOMEM;
+  const size_t size[4] = {sizeof(uint4) * s.mat_stride * all, sizeof(short) * 32 * s.strips * all,
+                          sizeof(double) * s.ext_stride * all, group * chunk};
+  if (!spare_memory(h, size[0] + size[1] + size[2] + size[3])) return CHF_OK;
+  void* mem[4] = {};
+  auto drop = [&] {
+    for (void* p : mem) cudaFree(p);
+    cudaGetLastError();
+  };
+  for (int i = 0; i < 4; ++i)
+    if (cudaMalloc(&mem[i], size[i]) != cudaSuccess) {
+      drop();
+      return CHF_OK;
+    }
+  uint4* const mat = static_cast<uint4*>(mem[0]);
+  short* const exps = static_cast<short*>(mem[1]);
+  double *const ext = static_cast<double*>(mem[2]), *const minc = static_cast<double*>(mem[3]);
   const size_t smem = sizeof(double) * (size_t)s.n[0] * BW64;
   for (int g0 = 0; g0 < h->nk2; g0 += chunk) {
     const int ng = std::min(chunk, h->nk2 - g0);
     k_build_m64<<<dim3(ng, 4), 256, smem, h->stream>>>(h->t0, h->t2, h->t4, h->k2vals, h->xinv, h->sl, h->d.N,
                                                        h->cfg.dt / h->cfg.re, g0, minc);
-    k_digits_solve64<<<dim3(ng, s.strips), 256, 0, h->stream>>>(minc, h->xinv, h->sl, s, g0, h->s64_mat, h->s64_exp,
-                                                                h->s64_ext);
+    k_digits_solve64<<<dim3(ng, s.strips), 256, 0, h->stream>>>(minc, h->xinv, h->sl, s, g0, mat, exps, ext);
   }
-  const bool ok = cuda_ok(h, cudaGetLastError(), "solve set-up") &&
-                  cuda_ok(h, cudaStreamSynchronize(h->stream), "solve set-up");
+  // the (0,0) mode's inverse alone, in place of all
+  double* keep = nullptr;
+  if (cudaMalloc((void**)&keep, group) != cudaSuccess) {
+    drop();
+    return CHF_OK;
+  }
+  if (!cuda_ok(h, cudaGetLastError(), "solve set-up") ||
+      !cuda_ok(h, cudaMemcpyAsync(keep, h->xinv + h->sl.stride * all, group, cudaMemcpyDeviceToDevice, h->stream),
+               "solve set-up") ||
+      !cuda_ok(h, cudaStreamSynchronize(h->stream), "solve set-up")) {
+    drop();
+    cudaFree(keep);
+    return CHF_E_CUDA;
+  }
   cudaFree(minc);
-  return ok ? CHF_OK : CHF_E_CUDA;
+  cudaFree(h->xinv);
+  h->xinv = keep;
+  h->xinv_first = h->nk2;
+  h->s64 = s;
+  h->s64_mat = mat;
+  h->s64_exp = exps;
+  h->s64_ext = ext;
+  return CHF_OK;
 }
 
 int launch_solve64(Handle* h) {
