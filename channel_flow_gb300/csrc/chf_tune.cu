@@ -12,7 +12,9 @@
 //     2, 3, 5 for the wall-normal ones; the x / y lines also try radices up to 4;
 //   * the lines per CTA of the two-buffer FFT kernels (y: streamwise modes per
 //     CTA; x: rows per CTA; FP64 z: modes per CTA), every shape the launch
-//     rules accept, against the in-place kernels or digit products of the rule;
+//     rules accept, against the in-place kernels of the rule (FP32 x / y lines).
+//     CHF_FP64 lines that go through digit products (k_dft64.cu) have neither
+//     radices nor lines per CTA: nothing is timed for them;
 //   * the increment solve's thread mapping (CHF_MIXED): modes per CTA (2 or
 //     4), matrix columns per load batch (2, 3 or 4) and rows per thread (1 or 2).
 // Every candidate computes the same results bit for bit (a plan change
@@ -118,15 +120,32 @@ double time_steps(Handle* h, int nsteps, int reps, cudaEvent_t e0, cudaEvent_t e
   return best;
 }
 
+// whether the step's x / y or z lines go through digit products
+bool digit_xy(const Handle* h) { return !mixed_front(h) && tf_xy(h); }
+bool digit_z(const Handle* h) { return !mixed_front(h) && tf_z(h); }
+
 std::string describe(const Handle* h, double ms_rule, double ms_best) {
+  // what a step launches: no radices or shapes of lines in digit products
+  std::string radices, shapes;
+  if (digit_xy(h)) {
+    shapes += "x / y lines as digit products, ";
+  } else {
+    radices += "py " + radix_string(h->py) + " px " + radix_string(h->px) + " ";
+    shapes += "kxb " + std::to_string(h->tune.kxb) + " xr " + std::to_string(h->tune.xr) + " ";
+  }
+  radices += "pz2 " + radix_string(h->pz2);
+  if (digit_z(h)) {
+    shapes += "z lines as digit products";
+  } else {
+    radices += " pzm " + radix_string(h->pzm);
+    shapes += "zl_c2v " + std::to_string(h->tune.zl_c2v) + " zl_curl " + std::to_string(h->tune.zl_curl);
+  }
   char buf[512];
   std::snprintf(buf, sizeof buf,
-                "fft radices py %s px %s pz2 %s pzm %s; kxb %d xr %d zl_c2v %d zl_curl %d; "
+                "fft radices %s; %s; "
                 "increment solve %d modes x %d columns x %d rows per thread, %s recovery; step %.4f ms "
                 "(rules %.4f ms)",
-                radix_string(h->py).c_str(), radix_string(h->px).c_str(), radix_string(h->pz2).c_str(),
-                radix_string(h->pzm).c_str(), h->tune.kxb, h->tune.xr, h->tune.zl_c2v, h->tune.zl_curl,
-                inc_modes(h), h->tune.inc_cb, h->tune.inc_rpt,
+                radices.c_str(), shapes.c_str(), inc_modes(h), h->tune.inc_cb, h->tune.inc_rpt,
                 (h->tune.rec_form >= 0 ? h->tune.rec_form == 1 : h->rec_df_rule) ? "double-float" : "FP64", ms_best,
                 ms_rule);
   return buf;
@@ -212,7 +231,7 @@ int chf_autotune(chf_handle* h, int reps) {
   };
   bool tw_ok = true;
   const bool reg_xy = mixed_front(h) && xy_register_path(d);
-  if (!reg_xy) {
+  if (!reg_xy && !digit_xy(h)) {
     // two-buffer stages: the large-radix rule's orders, and radices up to 4
     const int maxr = h->cfg.precision == CHF_FP64 ? 8 : 16;
     auto xy_cands = [&](int L) {
@@ -228,7 +247,7 @@ int chf_autotune(chf_handle* h, int reps) {
     try_knob([&](int v) { h->tune.kxb = v; }, with_current(h->tune.kxb, shape_candidates(h, 0)));
     try_knob([&](int v) { h->tune.xr = v; }, with_current(h->tune.xr, shape_candidates(h, 1)));
   }
-  if (!mixed_front(h)) {
+  if (!mixed_front(h) && !digit_z(h)) {
     try_knob([&](const FftPlan& p) { h->pzm = p; }, with_current(h->pzm, plan_candidates(make_plan(2 * d.MZ))));
     try_knob([&](int v) { h->tune.zl_c2v = v; }, with_current(h->tune.zl_c2v, shape_candidates(h, 2)));
     try_knob([&](int v) { h->tune.zl_curl = v; }, with_current(h->tune.zl_curl, shape_candidates(h, 3)));
