@@ -312,7 +312,7 @@ int chf_set_launch_shape(chf_handle* h, const char* name, int value) {
     return CHF_E_INVALID;
   };
   if (n == "inc_modes") {
-    if (value != 2 && value != 4) return bad("2 or 4 modes per CTA");
+    if (value != 0 && value != 2 && value != 4) return bad("2 or 4 modes per CTA, or 0 for the rule");
     t.inc_mch = value;
   } else if (n == "inc_columns") {
     if (value < 2 || value > 4) return bad("2, 3 or 4 columns per batch");

@@ -363,7 +363,6 @@ __global__ void __launch_bounds__(THREADS, RPT == 2 ? 6 : MCH == 2 && THREADS <=
     if (threadIdx.x < MCH * 2) s_cexp[threadIdx.x] = 0;
     __syncthreads();
     // (mode, entry) loops without divisions by the run-time sizes
-    // (mode, entry) loops without divisions by the run-time sizes
     for (int q = 0; q < nm; ++q)
       for (int k = threadIdx.x; k < NZ; k += blockDim.x) {
         const cd x = C[(size_t)k * modes + s_mode[q]];

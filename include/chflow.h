@@ -197,7 +197,8 @@ int chf_tuning(const chf_handle* h, char* buf, int len);
 /* Sets one launch shape by name, in place of the rule or the autotuner's
  * choice (every shape but "recover_form" computes the same results, bit for
  * bit):
- *   "inc_modes"    modes per CTA of the CHF_MIXED increment solve: 2 or 4
+ *   "inc_modes"    modes per CTA of the CHF_MIXED increment solve: 2 or 4,
+ *                  or 0 for the launcher's rule
  *   "inc_columns"  its matrix columns per load batch: 2, 3 or 4
  *   "inc_rows"     its block rows per thread: 1 or 2 (2 with 2 or 3 columns)
  *   "inc_wide"     0 or 1, without effect: a block holds every row of its
