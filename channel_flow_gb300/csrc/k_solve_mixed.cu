@@ -789,17 +789,26 @@ int setup_inc_items(Handle* h) {
 
 // Modes per CTA.  Four read the operators and compute a row's exponent once
 // for more products; two, with half the shared memory and 56 registers a
-// thread, are shorter CTAs, which is better where there are few of them (under
-// 16 per SM), and let more threads run where a field fills five warps (129 to
-// 160 rows: 7 CTAs per SM against 5).  Two against four: 33 rows 12 / 15 us
-// (32 x 33 x 32), 96 channels of 33 to 97 rows one after another 133 / 136 us a
-// step, 129 rows 209 / 221 us (128 x 129 x 128); but 97 rows 160 / 158 us
-// (160 x 97 x 120), 193 rows 3245 / 3089 us (384 x 193 x 384), and the 96
-// channels stacked in six classes 56.7 / 55.4 us a channel-step.
+// thread instead of 72, are shorter CTAs and more of them.  What that gives
+// depends on how full the runs of four are, which is a matter of the box: n2
+// runs of two to n4 of four are 1 (a k^2 in one or two modes) to 2 (square
+// boxes).  Times of two over four, by rows and warps of a field's block:
+//   16 CTAs per SM and more: 129 to 192 rows (5 and 6 warps; 7 and 6 CTAs per
+//     SM against 5 and 4) 0.94 to 0.97 at n2 / n4 = 1.25 (128^2 and 192^2
+//     modes, box 4 pi x 4/3 pi), 1.005 to 1.013 at 1.45 (160 x 120, 384^2), 1.10
+//     to 1.13 at 1.97 (square); 193 rows and more 1.00 to 1.04, 1.06 and 1.10 to
+//     1.18.  Up to 128 rows 0.91 to 1.00, 0.93 to 1.02 and 1.01 to 1.12, but 96
+//     channels stacked in six classes 56.7 / 55.4 us a channel-step at 1.25;
+//   fewer: 0.62 to 1.00 at 1.09 to 1.25 (16^2, 32^2, 64 x 48 modes, 33 to 251
+//     rows); at 1.65 and 1.89 0.82 to 1.00 up to 160 rows (one of 1.05), 0.93
+//     to 1.14 above.
 int inc_modes(const Handle* h) {
   if (h->tune.inc_mch) return h->tune.inc_mch;
   const int NZ = h->d.NZ;
-  return NZ <= 160 && (NZ > 128 || 2 * h->n_inc_items[1] < 16 * h->num_sms) ? 2 : 4;
+  const long n2 = h->n_inc_items[0], n4 = h->n_inc_items[1];
+  const bool partial = 3 * n2 < 4 * n4;
+  if (2 * n4 < 16L * h->num_sms) return NZ <= 160 || partial ? 2 : 4;
+  return partial && NZ > 128 && NZ <= 192 ? 2 : 4;
 }
 
 int launch_recover(Handle* h, bool df) {
