@@ -25,13 +25,13 @@ __device__ __forceinline__ uint32_t to_half2(uint32_t w, uint32_t sel) {
   return *reinterpret_cast<const uint32_t*>(&r);
 }
 
-// x 2^(61 - e) rounded to an integer, |x| < 2^e, e = emax - 1022
+// x 2^(61 - e) rounded to an integer, |x| < 2^e, e = emax - 1022, emax >= 1
+// (zeros and subnormals have the exponent of 1, without its leading bit)
 __device__ __forceinline__ long long fixed_of(uint32_t lo, uint32_t hi, int emax) {
   const int ex = (int)((hi >> 20) & 0x7ffu);
-  if (ex == 0) return 0;  // zero (subnormals count as zero)
-  const int d = emax - ex;  // >= 0
+  const int d = emax - max(ex, 1);  // >= 0
   if (d > 62) return 0;
-  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 8;
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | (ex ? 0x100000u : 0u)) << 32 | lo) << 8;
   unsigned long long t = m >> d;
   if (d > 0) t += (m >> (d - 1)) & 1ull;
   return (int)hi < 0 ? -(long long)t : (long long)t;

@@ -97,10 +97,12 @@ __device__ __forceinline__ void digit_halves(const long long* x, uint32_t (&word
 }
 
 // t 2^n, the exponent added to the conversion's (n in the range where every
-// result is normal; `scale` serves the other lines)
+// result is normal; `scale` serves the other lines: the largest times 1, the
+// smallest, whose factor is no double, in two steps)
+constexpr int TF_LARGE = INT_MIN, TF_SMALL = INT_MIN + 1;
 __device__ __forceinline__ double scaled(long long t, int n, double scale) {
   const double v = (double)t;
-  if (n == INT_MIN) return v * scale;
+  if (n <= TF_SMALL) return n == TF_LARGE ? v * scale : t == 0 ? 0.0 : v * scale * 0x1p-200;
   return t == 0 ? 0.0 : __hiloint2double(__double2hiint(v) + (n << 20), __double2loint(v));
 }
 
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) k_tf(const __grid_constan
     return (plane * KS + (octet >> 1)) * 32 + (octet & 1) * 16 + slot;
   };
   if (tid < TF_LINES) {
-    s_emax[tid] = 0;
+    s_emax[tid] = 1;
     s_sum[tid] = 0u;
   }
   // ---- the values' bits into pieces of planes 0..3, the largest exponent
@@ -256,8 +258,8 @@ __global__ void __launch_bounds__(TF_THREADS, TF_CTAS) k_tf(const __grid_constan
     const int e = s_emax[tid];
     const int b = max(0, 32 - __clz(s_sum[tid]) - 21), n = e - 1022 + sh.f - 57 + b;
     s_shift[tid] = 10 + b;
-    s_exp[tid] = n > -960 && n < 900 ? n : INT_MIN;
-    s_scale[tid] = e == 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(1.0, n);
+    s_exp[tid] = n >= 900 ? TF_LARGE : n <= -960 ? TF_SMALL : n;
+    s_scale[tid] = e == 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(1.0, n <= -960 ? n + 200 : n);
   }
   __syncthreads();
   // ---- products: warp = every fourth tile of 8 outputs

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) k_solve64(const __grid_constan
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       const int par = t & 1, op = t >> 1, blk = 2 * f + par;
-      int e = 0;
+      int e = 1;
 #pragma unroll
       for (int i = 0; i < ITER; ++i)
 #pragma unroll
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(256) k_digits_solve64(const double* __restrict
   const size_t off = blk == 0 ? bo.ve : blk == 1 ? bo.vo : blk == 2 ? bo.we : bo.wo;
   const double* src[2] = {minc + (size_t)gl * sl.stride + off, xinv + (size_t)g * sl.stride + off};
   const int first[2] = {0, blk < 2 ? 2 : 1};  // A^-1's columns of the wall rows, whose r is zero, stay out
-  if (tid < 32) s_e[tid >> 4][tid & 15] = 0;
+  if (tid < 32) s_e[tid >> 4][tid & 15] = 1;
   __syncthreads();
   for (int op = 0; op < 2; ++op) {
     const int r = 16 * i + (tid & 15);
@@ -378,10 +378,10 @@ __global__ void __launch_bounds__(256) k_digits_solve64(const double* __restrict
     atomicMax(&s_e[op][tid & 15], e);
   }
   __syncthreads();
-  // a row's power of two; entries 2^-600 below are zero, rows of zeros take 0
+  // a row's power of two
   if (tid < 32)
     exps[(((size_t)g * sh.strips + s) * 8 + (tid & 7)) * 4 + 2 * ((tid >> 3) & 1) + (tid >> 4)] =
-        (short)(s_e[tid >> 4][tid & 15] ? s_e[tid >> 4][tid & 15] - 1022 : 0);
+        (short)(s_e[tid >> 4][tid & 15] - 1022);
   uint4* out = mat + (size_t)g * sh.mat_stride + (size_t)(sh.mat0[blk] + 2 * T * i) * S64_BLOCK + lane;
   for (int t = warp; t < 2 * T; t += 8) {
     const int op = t / T, kt = t - op * T;
