@@ -23,8 +23,9 @@
 // (90 instructions; 293 -> 237 us there, 2264 -> 1822 us at 384 x 193 x 384,
 // 165 -> 138 us at 160 x 97 x 120).  More threads per SM at 56 registers spill
 // (2076 us at 384 x 193 x 384), and blocks sized to whole passes of the stages
-// change nothing (1822).  The y kernels have no swizzle; they run at 0.62 to
-// 0.66 of the memory rate at 384 x 193 x 384 (765 and 411 us).
+// change nothing (1822).  The y kernels have no swizzle; at 384 x 193 x 384
+// they take 765 us for 2.66 GB and 411 us for 1.33 GB, 0.51 and 0.48 of the
+// 6763 GB/s of a copy (loads' latency, and issue in 61 and 50% of the cycles).
 #include <algorithm>
 
 #include "chf_internal.h"

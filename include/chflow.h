@@ -41,15 +41,16 @@ extern "C" {
 #define CHF_E_STATE (-4)     /* call out of order (e.g. step before upload) */
 #define CHF_E_NUMERIC (-5)   /* non-finite values detected */
 
-#define CHF_FP64 0           /* all arithmetic in FP64 */
+#define CHF_FP64 0           /* FP64, or exact digit products of no larger error
+                                (transforms; the solve of grids with many modes) */
 #define CHF_MIXED 1          /* FP32 x/y transforms and products, exact tensor-core
                                 z transforms, FP64 state; the per-mode solve as an
                                 FP64 update c + delta whose increment delta is
                                 formed by compensated FP32 arithmetic (about
                                 2^-38 of its terms), A^-1 r in FP32; the (0,0)
                                 mode and the operator factorisations in FP64 */
-#define CHF_MIXED_F64SOLVE 2 /* the nonlinear term of CHF_MIXED with the FP64
-                                tau solve of CHF_FP64 for every mode */
+#define CHF_MIXED_F64SOLVE 2 /* the nonlinear term of CHF_MIXED with the tau solve
+                                of every mode on the FP64 pipe */
 
 /* Runtime counterpart of the compile-time parameters of paraandcons.f90:4-25. */
 typedef struct chf_config {
