@@ -128,15 +128,14 @@ __host__ __device__ __forceinline__ double widen(float f) {
   return u2d(sign | (ed << 52) | ((uint64_t)(v & 0x7fffffu) << 29));
 }
 
-// x / 2 on the bits, as x * 0.5 gives it: the exponent less one; infinity and
-// NaN stay what they are (less one they would be finite), and below 2^-1021 the
-// significand is halved instead, ties to even
+// x / 2 by decrementing the exponent (exact for |x| >= 2^-1021; smaller
+// magnitudes give signed zero).  Infinity and NaN stay what they are: one less
+// in the exponent they would be finite
 __host__ __device__ __forceinline__ double half(double x) {
-  const uint64_t u = d2u(x), m = u & 0x7fffffffffffffffull;
-  const int e = (int)(m >> 52);
-  if (e == 0x7ff) return x;
-  if (e > 1) return u2d(u - (1ull << 52));
-  return u2d((u & 0x8000000000000000ull) | ((m >> 1) + ((m >> 1) & m & 1)));
+  const uint64_t u = d2u(x);
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+  if (e - 2u < 0x7fdu) return u2d(u - (1ull << 52));
+  return e == 0x7ffu ? x : u2d(u & 0x8000000000000000ull);
 }
 
 // the binary64 of an integer 1 <= n < 2^31 (exact)
