@@ -128,14 +128,14 @@ __host__ __device__ __forceinline__ double widen(float f) {
   return u2d(sign | (ed << 52) | ((uint64_t)(v & 0x7fffffu) << 29));
 }
 
-// x / 2 by decrementing the exponent (exact for |x| >= 2^-1021; smaller
-// magnitudes give signed zero).  Infinity and NaN stay what they are: one less
-// in the exponent they would be finite
+// x / 2 by decrementing the exponent, exact for |x| >= 2^-1021.  Infinity and
+// NaN stay what they are (one less in the exponent, they would be finite), and so
+// do smaller magnitudes.
 __host__ __device__ __forceinline__ double half(double x) {
   const uint64_t u = d2u(x);
-  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
-  if (e - 2u < 0x7fdu) return u2d(u - (1ull << 52));
-  return e == 0x7ffu ? x : u2d(u & 0x8000000000000000ull);
+  const uint32_t hi = (uint32_t)(u >> 32);
+  const uint32_t less = (hi & 0x7ff00000u) - 0x00200000u < 0x7fd00000u ? 0x00100000u : 0u;
+  return u2d((uint64_t)(hi - less) << 32 | (uint32_t)u);
 }
 
 // the binary64 of an integer 1 <= n < 2^31 (exact)
